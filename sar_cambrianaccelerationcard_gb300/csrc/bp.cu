@@ -26,6 +26,19 @@
 //    of sqrt(1+e); the planner bounds the truncation error) -- all on the FMA
 //    pipe; the phase fma(dR, k_hi, phi_T) + dR k_lo (compensated product); the
 //    only MUFU work is one sin/cos pair.
+//  * What bounds the pixel loop is the register file: a scheduler reads two
+//    32-lane registers per clock, so an FMA of three distinct registers takes
+//    1.3-1.5 clk and a packed FP32x2 FMA of three register pairs 3.1, not 2
+//    (microbenchmark; 2.6 with one operand a scalar read as both halves, 2.0
+//    with two).  So per-pulse constants enter the packed operations as scalars
+//    (not as stored pairs, which also halves their shared loads); the
+//    interpolation and the sums run packed over (re, im) of one pixel, on two
+//    accumulators, sum s cos and sum s sin, combined at the end, so neither
+//    the loaded pair nor the sample is repacked (3 instructions per update, 6
+//    before); and the staging buffer's address is part of the per-pulse
+//    rounding constant, so a pixel's shared address is one shift-add with an
+//    immediate.  Config 2 (4096 pulses, 4096^2 pixels) 52.9 -> 45.8 ms, FP16
+//    rows 9% and the linear-term form 8% faster, same phases bit for bit.
 //  * Staging windows are sized so every bin a pixel can need lies inside
 //    [1, win-3]; the producer checks this per (tile, pulse) and, should a pulse
 //    fail the check, neutralises it (no data, bin 1) and raises an error bit,
@@ -64,9 +77,11 @@ constexpr int kTileX = 32;  // pixels along x (columns); tile height is 8 * PIX 
 #define SARBP_BP_PHASE_COMPENSATED 0
 #endif
 #ifndef SARBP_BP_PULSE_UNROLL
-#define SARBP_BP_PULSE_UNROLL 2
+#define SARBP_BP_PULSE_UNROLL 4
 #endif
-constexpr int kPulseUnroll = SARBP_BP_PULSE_UNROLL;  // pulses per loop body (SPLIT)
+// pulses per loop body (SPLIT); config 2 / 0.75 m pixels at 1, 2, 4, 8 pulses:
+// 46.4, 46.7, 45.8, 45.3 / 1.88, 1.85, 1.83, 1.89 ms
+constexpr int kPulseUnroll = SARBP_BP_PULSE_UNROLL;
 constexpr int kChunk = SARBP_BP_CHUNK;  // pulses per staged chunk (a multiple of 8)
 constexpr int kPerWarp = kChunk / kWarps;  // pulses each warp prepares
 static_assert(kChunk % kWarps == 0 && kPerWarp <= 32, "chunk must split evenly over the warps");
@@ -75,11 +90,13 @@ constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23: adding it rounds to an int
 constexpr unsigned kMagicBitsShift4 = 0x4B400000u << 4;
 
 struct __align__(16) Prm {
-    // SPLIT: each constant twice, so a 16-byte load yields two packed f32x2 operands
-    float4 k0;     // SPLIT: c1, c1, c2, c2     FP32: apc x, y, z, bin offset
-    float4 k1;     // SPLIT: c3, c3, c4, c4
-    float4 k2;     // SPLIT: bin', bin', phT, phT
-    float4 k3;     // SPLIT: A, A, B, B
+    // back-projection, split arithmetic: each constant once (the packed
+    // operations read a scalar as both halves); projection: each constant twice,
+    // so a 16-byte load yields two packed operands
+    float4 k0;     // c1, c2, c3, c4      projection: c1, c1, c2, c2     FP32: apc x, y, z, bin offset
+    float4 k1;     // bin', phT, A, B     projection: c3, c3, c4, c4
+    float4 k2;     // LIN: PX, PY, 0, 0   projection: bin', bin', phT, phT
+    float4 k3;     // -                   projection: A, A, B, B
     double ax, ay, az;  // FP64: APC position
     double dr, dph;     // FP64: per-pulse range (m) and phase (rad) corrections
     int ws;        // first bin of the window
@@ -88,7 +105,7 @@ struct __align__(16) Prm {
     int need;      // (M, d) pairs [0, need) any pixel of the tile reads (the rest are not converted)
 };
 
-// Linear-term split (LIN) kernels: the phase increments per pixel step,
+// Linear-term projection: the phase increments per pixel step,
 // (PX, PX, PY, PY), in the 16 bytes of the FP64-only ax, ay (offset 64,
 // 16-byte aligned), so the record keeps its size.
 __device__ __forceinline__ float4 &prm_k4(Prm &q) { return *reinterpret_cast<float4 *>(&q.ax); }
@@ -130,10 +147,20 @@ __device__ __forceinline__ f2 fmul2(f2 a, f2 b) {
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
-// 16-byte shared load as two packed pairs
-__device__ __forceinline__ void lds2x2(const void *p, f2 &a, f2 &b) {
-    asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "r"(smem_addr(p)));
+// A scalar as both halves of a packed operand: read as one register, not two.
+__device__ __forceinline__ f2 bc2(float v) { return pk2(v, v); }
+// acc += a b.  The accumulator stays a float pair outside the instruction: as a
+// 64-bit loop variable it cost one register move per instruction and pulse body.
+__device__ __forceinline__ void ffma2_acc(float2 &acc, f2 a, f2 b) {
+    asm("{\n\t.reg .b64 d;\n\tmov.b64 d, {%0, %1};\n\tfma.rn.f32x2 d, %2, %3, d;\n\tmov.b64 {%0, %1}, d;\n\t}"
+        : "+f"(acc.x), "+f"(acc.y)
+        : "l"(a), "l"(b));
 }
+// 16-byte shared load as two packed pairs
+__device__ __forceinline__ void lds2x2_at(unsigned addr, f2 &a, f2 &b) {
+    asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "r"(addr));
+}
+__device__ __forceinline__ void lds2x2(const void *p, f2 &a, f2 &b) { lds2x2_at(smem_addr(p), a, b); }
 
 struct Smem {
     float4 *staged;      // [2][chunk][win]
@@ -212,7 +239,7 @@ __device__ __noinline__ void drain_after_timeout(const BpPlan &P, uint64_t *bars
 // one chunk.  Every warp arrives once on the stage's barrier.  `fault` (tests
 // only) arms warp 0's arrival with kFaultBytes that no copy delivers, so the
 // phase cannot complete and the consumers' bounded wait runs out.
-template <int MODE, int STORE, int PIX, bool LIN = false>
+template <int MODE, int STORE, int PIX, bool LIN, bool ADJ>
 __device__ __forceinline__ void produce(const BpPlan &P, const Smem &S, int stage, int p0, int count,
                                         const TileGeo &T, bool fault) {
     constexpr int kTileY = 8 * PIX;
@@ -283,11 +310,20 @@ __device__ __forceinline__ void produce(const BpPlan &P, const Smem &S, int stag
                     const ff kh = {0.5f * P.kp_h, 0.5f * P.kp_l};  // 2 pi fc / c
                     const float pxr = ff_mod_2pi(ff_mul(ff_mul(kh, uxw), invR));
                     const float pyr = ff_mod_2pi(ff_mul(ff_mul(kh, uyw), invR));
-                    q.k0 = make_float4(c1, c1, d2, d2);
-                    q.k1 = make_float4(d3, d3, d4, d4);
-                    q.k2 = make_float4(bb, bb, phT, phT);
-                    q.k3 = make_float4(A * c1, A * c1, B * c1, B * c1);
-                    prm_k4(q) = make_float4(pxr, pxr, pyr, pyr);
+                    if constexpr (ADJ) {
+                        q.k0 = make_float4(c1, c1, d2, d2);
+                        q.k1 = make_float4(d3, d3, d4, d4);
+                        q.k2 = make_float4(bb, bb, phT, phT);
+                        q.k3 = make_float4(A * c1, A * c1, B * c1, B * c1);
+                        prm_k4(q) = make_float4(pxr, pxr, pyr, pyr);
+                    } else {
+                        q.k0 = make_float4(c1, d2, d3, d4);
+                        q.k1 = make_float4(bb, phT, A * c1, B * c1);
+                        q.k2 = make_float4(pxr, pyr, 0.f, 0.f);
+                    }
+                } else if constexpr (!ADJ) {
+                    q.k0 = make_float4(c1, c2, c3, c4);
+                    q.k1 = make_float4(bb, phT, A, B);
                 } else {
                     q.k0 = make_float4(c1, c1, c2, c2);
                     q.k1 = make_float4(c3, c3, c4, c4);
@@ -627,6 +663,12 @@ __global__ void __launch_bounds__(kThreads, SARBP_BP_MINBLOCKS)
 #pragma unroll
     for (int j = 0; j < (MODE == SARBP_MODE_FP64 ? kPix : 1); ++j) { dacc_r[j] = 0.0; dacc_i[j] = 0.0; }
 
+    // back-projection sums, split arithmetic: sum of s cos(phase) and of s sin(phase)
+    constexpr bool kSplitBp = !ADJ && (MODE == SARBP_MODE_SPLIT || MODE == SARBP_MODE_FP16STORE);
+    float2 acc_c[kSplitBp ? kPix : 1], acc_s[kSplitBp ? kPix : 1];
+#pragma unroll
+    for (int j = 0; j < (kSplitBp ? kPix : 1); ++j) acc_c[j] = acc_s[j] = make_float2(0.f, 0.f);
+
     const float bpm = P.kb_h;
     const float kph_hi = P.kp_h, kph_lo = P.kp_l;  // 4 pi fc / c as a float pair
     const float wmax = (float)(win - 2);
@@ -669,7 +711,7 @@ __global__ void __launch_bounds__(kThreads, SARBP_BP_MINBLOCKS)
     const f2 X2C2 = pk2(2.f * xc, 2.f * xc);
 
     if (nchunks > 0)
-        produce<MODE, STORE, PIX, LIN>(P, S, 0, p_begin, min(chunk, p_end - p_begin), T, TESTF && P.fault_chunk == 0);
+        produce<MODE, STORE, PIX, LIN, ADJ>(P, S, 0, p_begin, min(chunk, p_end - p_begin), T, TESTF && P.fault_chunk == 0);
 
     bool failed = false;
     bool clamped = false;
@@ -682,7 +724,7 @@ __global__ void __launch_bounds__(kThreads, SARBP_BP_MINBLOCKS)
         const int count = min(chunk, p_end - pc0);
         if (c + 1 < nchunks) {
             const int pn = pc0 + chunk;
-            produce<MODE, STORE, PIX, LIN>(P, S, (c + 1) % kStages, pn, min(chunk, p_end - pn), T,
+            produce<MODE, STORE, PIX, LIN, ADJ>(P, S, (c + 1) % kStages, pn, min(chunk, p_end - pn), T,
                                       TESTF && P.fault_chunk == c + 1);
         }
         const bool ok =
@@ -717,19 +759,17 @@ __global__ void __launch_bounds__(kThreads, SARBP_BP_MINBLOCKS)
             // modulo 2 pi per pulse) plus 4 pi / lambda times the nonlinear remainder
             // qq c1 + m^2 poly(m), so no FP32 quantity of the size of the tile's
             // extent enters the phase
-            f2 MP = pk2(kMagic + (float)cen, kMagic + (float)cen);
-            const f2 WIN2 = pk2((float)win, (float)win);
+            float mp = kMagic + (float)(int)((smem_addr(stg) >> 4) + cen);  // the window middle's 16-byte slot
+            const float winf = (float)win;
 #pragma unroll kPulseUnroll
             for (int pl = 0; pl < count; ++pl) {
                 const Prm &q = S.prm[stage * kChunk + pl];
-                f2 C1, D2, D3, D4, BT, PHT, AP, BP, PX, PY;
-                lds2x2(&q.k0, C1, D2);
-                lds2x2(&q.k1, D3, D4);
-                lds2x2(&q.k2, BT, PHT);
-                lds2x2(&q.k3, AP, BP);
-                lds2x2(&prm_k4(q), PX, PY);
-                const f2 XAP = fmul2(XC2, AP);
-                const f2 PHX = ffma2(X2C2, PX, PHT);
+                const float4 v0 = lds128(smem_addr(&q.k0)), v1 = lds128(smem_addr(&q.k1));
+                const float2 v2 = *reinterpret_cast<const float2 *>(&q.k2);
+                const f2 C1 = bc2(v0.x), D2 = bc2(v0.y), D3 = bc2(v0.z), D4 = bc2(v0.w);
+                const f2 BT = bc2(v1.x), BP = bc2(v1.w), PY = bc2(v2.y);
+                const f2 XAP = bc2(xc * v1.z);
+                const f2 PHX = bc2(fmaf(2.f * xc, v2.x, v1.y));
 #pragma unroll
                 for (int h = 0; h < kPix / 2; ++h) {
                     const f2 qc = fmul2(QQ2[h], C1);
@@ -753,37 +793,35 @@ __global__ void __launch_bounds__(kThreads, SARBP_BP_MINBLOCKS)
                         }
                         b2 = pk2(bb[0], bb[1]);
                     }
-                    const f2 t2 = fadd2(b2, MP);
+                    const f2 t2 = fadd2(b2, bc2(mp));
                     float tt[2];
                     upk2(t2, tt[0], tt[1]);
 #pragma unroll
                     for (int u = 0; u < 2; ++u) {
                         const int j = 2 * h + u;
-                        const float4 v = lds128((__float_as_uint(tt[u]) << 4) + sbase);
-                        const float sr = fmaf(bb[u], v.z, v.x);
-                        const float si = fmaf(bb[u], v.w, v.y);
+                        f2 M, D;
+                        lds2x2_at((__float_as_uint(tt[u]) << 4) - kMagicBitsShift4, M, D);
+                        const f2 sv = ffma2(bc2(bb[u]), D, M);
                         float sn, cs;
                         __sincosf(ph[u], &sn, &cs);
-                        acc_r[j] = fmaf(sr, cs, fmaf(-si, sn, acc_r[j]));
-                        acc_i[j] = fmaf(sr, sn, fmaf(si, cs, acc_i[j]));
+                        ffma2_acc(acc_c[j], sv, bc2(cs));
+                        ffma2_acc(acc_s[j], sv, bc2(sn));
                     }
                 }
-                MP = fadd2(MP, WIN2);
+                mp += winf;
             }
         } else if (MODE == SARBP_MODE_SPLIT || MODE == SARBP_MODE_FP16STORE) {
             // geometry, bin and phase for pixel pairs (2j, 2j+1) in packed FP32x2;
             // interpolation and the complex accumulate per pixel
-            f2 MP = pk2(kMagic + (float)cen, kMagic + (float)cen);
-            const f2 WIN2 = pk2((float)win, (float)win);
+            float mp = kMagic + (float)(int)((smem_addr(stg) >> 4) + cen);  // the window middle's 16-byte slot
+            const float winf = (float)win;
 #pragma unroll kPulseUnroll
             for (int pl = 0; pl < count; ++pl) {
                 const Prm &q = S.prm[stage * kChunk + pl];
-                f2 C1, C2, C3, C4, BT, PHT, AA, BB;
-                lds2x2(&q.k0, C1, C2);
-                lds2x2(&q.k1, C3, C4);
-                lds2x2(&q.k2, BT, PHT);
-                lds2x2(&q.k3, AA, BB);
-                const f2 XA = fmul2(XC2, AA);
+                const float4 v0 = lds128(smem_addr(&q.k0)), v1 = lds128(smem_addr(&q.k1));
+                const f2 C1 = bc2(v0.x), C2 = bc2(v0.y), C3 = bc2(v0.z), C4 = bc2(v0.w);
+                const f2 BT = bc2(v1.x), PHT = bc2(v1.y), BB = bc2(v1.w);
+                const f2 XA = bc2(xc * v1.z);
 #pragma unroll
                 for (int h = 0; h < kPix / 2; ++h) {
                     const f2 n = ffma2(YC2[h], BB, fadd2(XA, QQ2[h]));
@@ -810,22 +848,22 @@ __global__ void __launch_bounds__(kThreads, SARBP_BP_MINBLOCKS)
                         }
                         b2 = pk2(bb[0], bb[1]);
                     }
-                    const f2 t2 = fadd2(b2, MP);
+                    const f2 t2 = fadd2(b2, bc2(mp));
                     float tt[2];
                     upk2(t2, tt[0], tt[1]);
 #pragma unroll
                     for (int u = 0; u < 2; ++u) {
                         const int j = 2 * h + u;
-                        const float4 v = lds128((__float_as_uint(tt[u]) << 4) + sbase);
-                        const float sr = fmaf(bb[u], v.z, v.x);
-                        const float si = fmaf(bb[u], v.w, v.y);
+                        f2 M, D;
+                        lds2x2_at((__float_as_uint(tt[u]) << 4) - kMagicBitsShift4, M, D);
+                        const f2 sv = ffma2(bc2(bb[u]), D, M);
                         float sn, cs;
                         __sincosf(ph[u], &sn, &cs);
-                        acc_r[j] = fmaf(sr, cs, fmaf(-si, sn, acc_r[j]));
-                        acc_i[j] = fmaf(sr, sn, fmaf(si, cs, acc_i[j]));
+                        ffma2_acc(acc_c[j], sv, bc2(cs));
+                        ffma2_acc(acc_s[j], sv, bc2(sn));
                     }
                 }
-                MP = fadd2(MP, WIN2);
+                mp += winf;
             }
         } else if (MODE == SARBP_MODE_FP32) {
 #pragma unroll 1
@@ -898,6 +936,14 @@ __global__ void __launch_bounds__(kThreads, SARBP_BP_MINBLOCKS)
             flush_projection(P, S, last & 1, p_begin + last * chunk, min(chunk, p_end - p_begin - last * chunk));
         }
         return;
+    }
+
+    if constexpr (kSplitBp) {  // s e^{j phase}: (s.x cos - s.y sin, s.y cos + s.x sin)
+#pragma unroll
+        for (int j = 0; j < kPix; ++j) {
+            acc_r[j] = acc_c[j].x - acc_s[j].y;
+            acc_i[j] = acc_c[j].y + acc_s[j].x;
+        }
     }
 
     // write the tile
