@@ -8,9 +8,8 @@
 // loads, sqrtf + sincosf per pulse).
 //
 // Design (one CTA per TILE_X x TILE_Y pixel tile, optionally per pulse segment):
-//  * Pulses are processed in chunks of CHUNK.  For each chunk every warp
-//    computes, for two of its pulses, the tile-centre reference: range R_T
-//    (FP32 square root refined by one FP64 Newton step), the FP64-wrapped
+//  * Pulses are processed in chunks of CHUNK.  For each chunk one staging warp
+//    computes, a lane per pulse, the tile-centre reference: range R_T, wrapped
 //    carrier phase, the bin of the tile centre and the window of bins the tile
 //    can touch; it then issues one TMA bulk copy (cp.async.bulk, local HBM ->
 //    shared memory, completion on an mbarrier) per pulse for that window.  A
@@ -20,6 +19,21 @@
 //    mid_i = (s_i + s_{i+1})/2, diff_i = s_{i+1} - s_i, so one 16-byte shared load
 //    and two FMAs interpolate.  Converted windows are double-buffered: one
 //    block barrier per chunk.
+//  * Who stages (helper_warps): with 16-pulse chunks of 32 x 64 tiles, two extra
+//    warps per CTA, beside the pixel warps' loop over the chunk before.  The
+//    parameters (a float-float chain of some 400 instructions) then run once per
+//    chunk instead of in every warp, and neither they nor the conversion hold
+//    the pixel warps at the barrier.  20 warps per SM leave 96 registers, which
+//    the pixel loop needs: config 2 45.8 -> 42.6 ms, FP16 rows 3.63 -> 3.42 ms
+//    (the warps taking turns at the parameters, everyone converting: 44.8 and
+//    3.49 ms), weighted projection 1.78 -> 1.71 ms.  Where a chunk has less pixel
+//    work per staged bin (8 and 4 pulses, shorter tiles: wide windows) two warps
+//    cannot keep up, and the linear-term back-projection needs more than 96
+//    registers; there, and in the checked and comparator kernels, the pixel
+//    warps stage, each chunk's parameters by the next warp in turn.  1024 pulses
+//    onto 1024^2, helpers / none: 1.0 m pixels 1.40 / 1.35 ms, 1.4 m rotated by
+//    45 degrees 3.84 / 3.11 (3.81 before), 2.2 m onto 512^2 2.08 / 1.54 (1.85
+//    before), linear-term 0.5 m FP16 rows 1.03 / 1.00 (1.19 before).
 //  * SPLIT arithmetic per pixel and pulse: with q the pixel offset from the tile
 //    centre, n = 2 q.w + |q|^2 (w = tile centre - APC) and the differential
 //    range dR = sqrt(R_T^2 + n) - R_T = n (c1 + n (c2 + n (c3 + n c4))) (series
@@ -76,15 +90,15 @@ constexpr int kTileX = 32;  // pixels along x (columns); tile height is 8 * PIX 
 #ifndef SARBP_BP_PHASE_COMPENSATED
 #define SARBP_BP_PHASE_COMPENSATED 0
 #endif
-#ifndef SARBP_BP_PULSE_UNROLL
-#define SARBP_BP_PULSE_UNROLL 4
-#endif
-// pulses per loop body (SPLIT); config 2 / 0.75 m pixels at 1, 2, 4, 8 pulses:
-// 46.4, 46.7, 45.8, 45.3 / 1.88, 1.85, 1.83, 1.89 ms
-constexpr int kPulseUnroll = SARBP_BP_PULSE_UNROLL;
 constexpr int kChunk = SARBP_BP_CHUNK;  // pulses per staged chunk (a multiple of 8)
-constexpr int kPerWarp = kChunk / kWarps;  // pulses each warp prepares
-static_assert(kChunk % kWarps == 0 && kPerWarp <= 32, "chunk must split evenly over the warps");
+// Staging warps of a CTA beside its kWarps pixel warps; 0: the pixel warps stage.
+template <int MODE, bool CHECKED, int PIX, bool ADJ, int CHUNK, bool LIN>
+__host__ __device__ constexpr int helper_warps() {
+    return !CHECKED && (MODE == SARBP_MODE_SPLIT || MODE == SARBP_MODE_FP16STORE) && PIX == 8 && CHUNK && (ADJ || !LIN)
+               ? 2
+               : 0;
+}
+static_assert(kChunk <= 32, "one staging lane per pulse of a chunk");
 constexpr int kStages = 3;  // raw-window ring depth
 constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23: adding it rounds to an integer
 constexpr unsigned kMagicBitsShift4 = 0x4B400000u << 4;
@@ -156,7 +170,15 @@ __device__ __forceinline__ void ffma2_acc(float2 &acc, f2 a, f2 b) {
         : "+f"(acc.x), "+f"(acc.y)
         : "l"(a), "l"(b));
 }
-// 16-byte shared load as two packed pairs
+__device__ __forceinline__ f2 fsub2(f2 a, f2 b) {
+    f2 d;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+// 16-byte shared store and load of two packed pairs
+__device__ __forceinline__ void sts2x2(void *p, f2 a, f2 b) {
+    asm volatile("st.shared.v2.b64 [%0], {%1, %2};" ::"r"(smem_addr(p)), "l"(a), "l"(b) : "memory");
+}
 __device__ __forceinline__ void lds2x2_at(unsigned addr, f2 &a, f2 &b) {
     asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "r"(addr));
 }
@@ -218,8 +240,8 @@ __global__ void pulse_ref_kernel(const double *__restrict__ apc, int np, BpGeom 
 }
 
 // After the wait for chunk c ran out: raise the timeout bit and let the copies
-// still in flight land before the CTA's shared memory is released.  Every warp
-// has issued chunks c and (if it exists) c + 1 and waited for all before them,
+// still in flight land before the CTA's shared memory is released.  The staging
+// warps have issued chunks c and (if it exists) c + 1 and waited for all before them,
 // so those two phases are the outstanding ones: wait for each on its own
 // parity (chunk k is phase k / kStages of ring stage k % kStages).  Out of line:
 // inlined, this cold path moved the main loop's schedule (config 2: 54.1 ms
@@ -235,22 +257,21 @@ __device__ __noinline__ void drain_after_timeout(const BpPlan &P, uint64_t *bars
     }
 }
 
-// Per-(tile, pulse) geometry, window and TMA issue for this warp's pulses of
-// one chunk.  Every warp arrives once on the stage's barrier.  `fault` (tests
-// only) arms warp 0's arrival with kFaultBytes that no copy delivers, so the
-// phase cannot complete and the consumers' bounded wait runs out.
+// Per-(tile, pulse) geometry, window and TMA issue for the pulses of one chunk,
+// by one warp (a lane per pulse), which arrives once on the stage's barrier.
+// `fault` (tests only) arms the arrival with kFaultBytes that no copy delivers,
+// so the phase cannot complete and the staging warps' bounded wait runs out.
 template <int MODE, int STORE, int PIX, bool LIN, bool ADJ>
 __device__ __forceinline__ void produce(const BpPlan &P, const Smem &S, int stage, int p0, int count,
                                         const TileGeo &T, bool fault) {
     constexpr int kTileY = 8 * PIX;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int slot = threadIdx.x & 31;
     const int win = P.win;
     const int esize = STORE == SARBP_STORE_C64 ? 8 : 4;
-    const int slot = warp * kPerWarp + lane;
     unsigned bytes = 0;
     const char *src = nullptr;
     unsigned dst = 0;
-    if (lane < kPerWarp && slot < count) {
+    if (slot < count) {
         const int p = p0 + slot;
         const float bpm = P.kb_h;  // bins per metre of range
         const float hx = 0.5f * (kTileX - 1), hy = 0.5f * (kTileY - 1);
@@ -383,24 +404,25 @@ __device__ __forceinline__ void produce(const BpPlan &P, const Smem &S, int stag
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
     const unsigned bar = smem_addr(&S.bar[stage]);
-    if (fault && warp == 0) total += kFaultBytes;
-    if (lane == 0) mbar_expect_tx_arrive(bar, total);
+    if (fault) total += kFaultBytes;
+    __syncwarp();  // the arrival below publishes every lane's parameters
+    if (slot == 0) mbar_expect_tx_arrive(bar, total);
     __syncwarp();
     if (bytes) tma_bulk_g2s(dst, src, bytes, bar);
 }
 
-// raw window -> (mid, diff) pairs; bins outside [lo, hi) read as zero.
-// Flat over (pulse, bin), used for complex64 rows.
-template <int MODE, int STORE, bool TRIM>
+// raw window -> (mid, diff) pairs; bins outside [lo, hi) read as zero.  By the
+// staging warps, flat over (pulse, bin), the whole window: the checked build
+// and the FP32 / FP64 comparators clamp reads anywhere in it.
+template <int MODE, int STORE>
 __device__ __forceinline__ void convert_flat(const Smem &S, int stage, int sbuf, int count, int win, unsigned win_magic,
-                                        int chunk) {
+                                             int chunk, int stager, int stagers) {
     const int total = count * win;
     float4 *st = S.staged + (size_t)sbuf * chunk * win;
-    for (int e = threadIdx.x; e < total; e += kThreads) {
+    for (int e = 32 * stager + (threadIdx.x & 31); e < total; e += 32 * stagers) {
         const int pl = (int)__umulhi((unsigned)e, win_magic);
         const int i = e - pl * win;
         const Prm &q = S.prm[stage * kChunk + pl];
-        if (TRIM && i >= q.need) continue;  // no pixel of the tile reads it
         const int lo = q.lo, hi = q.hi;
         const unsigned char *rw = S.raw + ((size_t)stage * chunk + pl) * win * raw_esize(STORE);
         float2 a = make_float2(0.f, 0.f), b = make_float2(0.f, 0.f);
@@ -423,65 +445,53 @@ __device__ __forceinline__ void convert_flat(const Smem &S, int stage, int sbuf,
     }
 }
 
-// The same with one warp per pulse (pulse-uniform bounds and scale, lane =
-// bin) and an unconditional path when the whole window was copied (every pulse
-// but those at the swath edges), used for complex16 rows.
-template <int MODE, int STORE, bool TRIM>
-__device__ __forceinline__ void convert_warp(const Smem &S, int stage, int sbuf, int count, int win, int chunk) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int cen = win >> 1;
-    float4 *stb = S.staged + (size_t)sbuf * chunk * win;
-    for (int pl = warp; pl < count; pl += kWarps) {
+// One stored bin as a packed (re, im) pair, FP16 rows times the pulse's scale.
+template <int STORE>
+__device__ __forceinline__ f2 raw_bin(const unsigned char *row, int i, f2 scale) {
+    if constexpr (STORE == SARBP_STORE_C64) {
+        return *reinterpret_cast<const f2 *>(row + 8 * i);
+    } else {
+        const float2 v = __half22float2(*reinterpret_cast<const __half2 *>(row + 4 * i));
+        return fmul2(pk2(v.x, v.y), scale);
+    }
+}
+
+// The same pairs for the unchecked SPLIT / FP16STORE kernels: a staging warp
+// per pulse, packed over (re, im), and only the pairs [0, need - 1) the tile
+// reads (bins [0, need); the checked build flags any read past need - 2).
+// Windows that lie inside the row, all but those at the swath edges, skip
+// the bounds tests.
+template <int STORE>
+__device__ __forceinline__ void convert_pulses(const Smem &S, int stage, int sbuf, int count, int win, int chunk,
+                                               int stager, int stagers) {
+    const int lane = threadIdx.x & 31;
+    for (int pl = stager; pl < count; pl += stagers) {
         const Prm &q = S.prm[stage * kChunk + pl];
-        const int lo = q.lo, hi = q.hi;
-        const float sc = STORE == SARBP_STORE_C32H ? q.scale : 1.f;
-        const unsigned char *rw = S.raw + ((size_t)stage * chunk + pl) * win * raw_esize(STORE);
-        float4 *st = stb + (size_t)pl * win;
-        const bool whole = lo == 0 && hi == win;
-        const int n = TRIM ? q.need : win;  // pairs any pixel of the tile reads
-        for (int i = lane; i < n; i += 32) {
-            float2 a = make_float2(0.f, 0.f), b = make_float2(0.f, 0.f);
-            const bool ina = whole || (i >= lo && i < hi);
-            const bool inb = whole ? i + 1 < win : (i + 1 >= lo && i + 1 < hi);
-            if (STORE == SARBP_STORE_C64) {
-                const float2 *r = reinterpret_cast<const float2 *>(rw);
-                if (ina) a = r[i];
-                if (inb) b = r[i + 1];
-            } else {
-                const __half2 *r = reinterpret_cast<const __half2 *>(rw);
-                if (ina) a = __half22float2(r[i]);
-                if (inb) b = __half22float2(r[i + 1]);
-                a.x *= sc; a.y *= sc; b.x *= sc; b.y *= sc;
-            }
-            const float dx = b.x - a.x, dy = b.y - a.y;
-            // FP32 arithmetic: pairs centred on the window middle, so that s = M + b d
-            // takes the centred position b directly; FP64 keeps (mid, diff).
-            const float o = MODE == SARBP_MODE_FP64 ? 0.f : (float)(i - cen);
-            st[i] = make_float4(fmaf(-o, dx, 0.5f * (a.x + b.x)), fmaf(-o, dy, 0.5f * (a.y + b.y)), dx, dy);
+        const int lo = q.lo, hi = q.hi, n = q.need - 1;
+        const f2 scale = bc2(STORE == SARBP_STORE_C32H ? q.scale : 1.f);
+        const unsigned char *row = S.raw + ((size_t)stage * chunk + pl) * win * raw_esize(STORE);
+        float4 *st = S.staged + ((size_t)sbuf * chunk + pl) * win;
+        float o = (float)((win >> 1) - lane);  // from the pair to the window middle
+        auto store = [&](int i, f2 a, f2 b) {
+            const f2 d = fsub2(b, a);
+            sts2x2(st + i, ffma2(bc2(o), d, fmul2(bc2(0.5f), fadd2(a, b))), d);
+        };
+        if (lo == 0 && hi > n) {
+#pragma unroll 1
+            for (int i = lane; i < n; i += 32, o -= 32.f)
+                store(i, raw_bin<STORE>(row, i, scale), raw_bin<STORE>(row, i + 1, scale));
+        } else {
+#pragma unroll 1
+            for (int i = lane; i < n; i += 32, o -= 32.f)
+                store(i, i >= lo && i < hi ? raw_bin<STORE>(row, i, scale) : 0ull,
+                      i + 1 >= lo && i + 1 < hi ? raw_bin<STORE>(row, i + 1, scale) : 0ull);
         }
     }
 }
 
-// Measured per storage on config 2 (Gupd/s, flat / warp-per-pulse): complex64
-// 1275.7 / 1241.5, complex16 1231.5 / 1244.8.  The pass itself is ~6% of the
-// kernel (3.1 ms of 53.9 without it), but its code shape moves the schedule
-// of the main loop more than its own cost.
-// TRIM: convert only the pairs [0, need) the tile reads (unchecked SPLIT /
-// FP16STORE kernels); the checked build and the FP32 / FP64 comparators clamp
-// reads anywhere in the window and convert all of it.
-template <int MODE, int STORE, bool TRIM>
-__device__ __forceinline__ void convert(const Smem &S, int stage, int sbuf, int count, int win, unsigned win_magic,
-                                        int chunk) {
-    if constexpr (STORE == SARBP_STORE_C32H)
-        convert_warp<MODE, STORE, TRIM>(S, stage, sbuf, count, win, chunk);
-    else
-        convert_flat<MODE, STORE, TRIM>(S, stage, sbuf, count, win, win_magic, chunk);
-}
-
 // Sum of the warps' projections for the pulses of one chunk into
 // proj[tile][pulse] (fixed order: deterministic).
-__device__ __forceinline__ void flush_projection(const BpPlan &P, const Smem &S, int buf, int p0, int count) {
-    const int t = threadIdx.x;
+__device__ __forceinline__ void flush_projection(const BpPlan &P, const Smem &S, int buf, int p0, int count, int t) {
     if (t < count) {
         float sr = 0.f, si = 0.f;
 #pragma unroll
@@ -597,13 +607,19 @@ __device__ __forceinline__ void project_chunk(const Smem &S, int stage, int coun
 // sarbp_debug_set); production variants wait 2 s and carry no injector.
 template <int MODE, int STORE, int NTERMS, bool CHECKED, int PIX, bool ADJ = false, int CHUNK = 0, bool TESTF = false,
           bool LIN = false>
-__global__ void __launch_bounds__(kThreads, SARBP_BP_MINBLOCKS)
+__global__ void __launch_bounds__(kThreads + 32 * helper_warps<MODE, CHECKED, PIX, ADJ, CHUNK, LIN>(), SARBP_BP_MINBLOCKS)
     bp_kernel(const __grid_constant__ BpPlan P, int tiles_y, int pulses_per_seg, float qq_max) {
     static_assert(!ADJ || MODE == SARBP_MODE_SPLIT || MODE == SARBP_MODE_FP16STORE, "projection: split arithmetic");
     static_assert(!LIN || MODE == SARBP_MODE_SPLIT || MODE == SARBP_MODE_FP16STORE,
                   "linear-term phase: split arithmetic only");
     constexpr int kPix = PIX;  // pixels per thread, all in one column
     constexpr int kTileY = 8 * PIX;
+    // pulses per loop body: series form with 16-pulse chunks 2 / 4 / 8 / 16: 43.7 / 43.5 /
+    // 43.6 / 42.6 ms at config 2; the others 1 / 2 / 4 / 8: 1.69 / 1.67 / 1.64 / 1.71 ms for
+    // the linear-term form at 0.75 m, 1.38 / 1.38 / 1.35 / 1.40 at 1 m
+    constexpr int kPulseUnroll = CHUNK && !LIN ? CHUNK : 4;
+    constexpr int kHelpers = helper_warps<MODE, CHECKED, PIX, ADJ, CHUNK, LIN>();
+    constexpr int kStager0 = kHelpers ? kWarps : 0, kStagers = kHelpers ? kHelpers : kWarps;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int win = P.win;
     const int chunk = CHUNK ? CHUNK : P.chunk;  // pulses per staged chunk: 16, 8 or 4 (two CTAs per SM)
@@ -640,7 +656,7 @@ __global__ void __launch_bounds__(kThreads, SARBP_BP_MINBLOCKS)
         T.xT = (float)pcx_i;
         T.yT = (float)pcy_i;
         T.qqh = T.qql = 0.f;
-        if (lane < kPerWarp) {  // producer lanes only: FP64 once per CTA
+        if (warp >= kStager0) {  // staging warps only: FP64 once per CTA
             const double qq = pcx_i * pcx_i * P.g.g11 + 2.0 * pcx_i * pcy_i * P.g.g12 + pcy_i * pcy_i * P.g.g22;
             T.qqh = (float)qq;
             T.qql = (float)(qq - (double)T.qqh);
@@ -650,7 +666,7 @@ __global__ void __launch_bounds__(kThreads, SARBP_BP_MINBLOCKS)
     const float cenf = (float)cen;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kStages; ++s) mbar_init(smem_addr(&S.bar[s]), kWarps);
+        for (int s = 0; s < kStages; ++s) mbar_init(smem_addr(&S.bar[s]), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -698,7 +714,7 @@ __global__ void __launch_bounds__(kThreads, SARBP_BP_MINBLOCKS)
         }
     }
 
-    const f2 XC2 = pk2(xc, xc);
+    const f2 XC2 = bc2(xc);
     const f2 BPM2 = pk2(bpm, bpm), KH2 = pk2(kph_hi, kph_hi), KL2 = pk2(kph_lo, kph_lo);
     f2 YC2[kPix / 2], QQ2[kPix / 2], TH2[ADJ ? kPix / 2 : 1], Y2C2[LIN ? kPix / 2 : 1];
 #pragma unroll
@@ -710,44 +726,58 @@ __global__ void __launch_bounds__(kThreads, SARBP_BP_MINBLOCKS)
     }
     const f2 X2C2 = pk2(2.f * xc, 2.f * xc);
 
-    if (nchunks > 0)
-        produce<MODE, STORE, PIX, LIN, ADJ>(P, S, 0, p_begin, min(chunk, p_end - p_begin), T, TESTF && P.fault_chunk == 0);
+    // Staging of chunk k: one staging warp computes the parameters and issues the
+    // copies of chunk k + 1, then all of them wait for chunk k's copies and
+    // convert them.  False when the wait ran out.
+    const bool helper = kHelpers && warp >= kWarps;
+    auto produce_chunk = [&](int k) {
+        const int p0 = p_begin + k * chunk;
+        if (k < nchunks && warp == kStager0 + (kHelpers ? 0 : k % kWarps))
+            produce<MODE, STORE, PIX, LIN, ADJ>(P, S, k % kStages, p0, min(chunk, p_end - p0), T,
+                                                TESTF && P.fault_chunk == k);
+    };
+    auto stage_chunk = [&](int k) {
+        produce_chunk(k + 1);
+        if (!mbar_wait_bounded(smem_addr(&S.bar[k % kStages]), (k / kStages) & 1, TESTF ? P.wait_ns : kDefaultWaitNs))
+            return false;
+        const int count = min(chunk, p_end - p_begin - k * chunk);
+        if constexpr (!CHECKED && (MODE == SARBP_MODE_SPLIT || MODE == SARBP_MODE_FP16STORE))
+            convert_pulses<STORE>(S, k % kStages, k & 1, count, win, chunk, warp - kStager0, kStagers);
+        else
+            convert_flat<MODE, STORE>(S, k % kStages, k & 1, count, win, win_magic, chunk, warp - kStager0, kStagers);
+        return true;
+    };
 
     bool failed = false;
     bool clamped = false;
+    if (warp >= kStager0) {
+        produce_chunk(0);
+        if (kHelpers && nchunks > 0) failed = !stage_chunk(0);
+    }
+    if (kHelpers) failed = __syncthreads_or(failed);
+    // One block barrier per chunk.  Helpers stage chunk c + 1 beside the pixel
+    // warps' chunk c and the barrier ends both; without helpers it follows chunk
+    // c's own staging.  Either way, when chunk k's copies and parameters are
+    // issued every warp is done with chunk k - 3 (the ring stage), and when its
+    // pairs are written with chunk k - 2 (the buffer).  A wait that ran out ends
+    // the loop for every warp.
     int c = 0;  // after a failed wait, the chunk it was for
 #pragma unroll 1
-    for (; c < nchunks; ++c) {
+    for (; c < nchunks && !failed; ++c) {
         const int stage = c % kStages;
         const int sbuf = c & 1;
         const int pc0 = p_begin + c * chunk;
         const int count = min(chunk, p_end - pc0);
-        if (c + 1 < nchunks) {
-            const int pn = pc0 + chunk;
-            produce<MODE, STORE, PIX, LIN, ADJ>(P, S, (c + 1) % kStages, pn, min(chunk, p_end - pn), T,
-                                      TESTF && P.fault_chunk == c + 1);
+        if constexpr (!kHelpers) {
+            failed = __syncthreads_or(!stage_chunk(c));
+            if (failed) break;
         }
-        const bool ok =
-            mbar_wait_bounded(smem_addr(&S.bar[stage]), (c / kStages) & 1, TESTF ? P.wait_ns : kDefaultWaitNs);
-        if (!ok) { failed = true; }
-        // One block barrier per chunk, after the conversion: each thread has seen
-        // its own wait complete, the chunk's parameters were published by the
-        // previous chunk's barrier, and a thread whose wait ran out converts
-        // in-bounds shared memory only before the barrier's vote ends the loop
-        // (config 2 53.04 -> 52.64 ms against a barrier on each side, same bits).
-        // trimmed to the pairs the tile reads for complex16 rows (warp per pulse:
-        // config 5 892 -> 864 ms); the flat complex64 pass measured slower with
-        // the per-element test (config 2 1296 -> 1283 Gupd/s), and complex64 rows
-        // through the trimmed warp-per-pulse pass tied with it (1300.2 vs
-        // 1301-1303), so complex64 converts the whole window
-        convert<MODE, STORE,
-                !CHECKED && STORE == SARBP_STORE_C32H && (MODE == SARBP_MODE_SPLIT || MODE == SARBP_MODE_FP16STORE)>(
-            S, stage, sbuf, count, win, win_magic, chunk);
-        if (__syncthreads_or(failed)) { failed = true; break; }
-        if constexpr (ADJ) {  // every warp has finished chunk c-1: combine its pulse sums
-            if (c > 0) flush_projection(P, S, (c - 1) & 1, pc0 - chunk, chunk);
+        if constexpr (ADJ) {  // every pixel warp has finished chunk c - 1: combine its pulse sums
+            if (c > 0 && warp == kStager0) flush_projection(P, S, (c - 1) & 1, pc0 - chunk, chunk, lane);
         }
-
+        if (helper) {
+            if (c + 1 < nchunks) failed = !stage_chunk(c + 1);
+        } else {
         const float4 *stg = S.staged + (size_t)sbuf * chunk * win;
         const unsigned sbase = smem_addr(stg) - kMagicBitsShift4;
         if constexpr (ADJ) {
@@ -768,12 +798,12 @@ __global__ void __launch_bounds__(kThreads, SARBP_BP_MINBLOCKS)
                 const float2 v2 = *reinterpret_cast<const float2 *>(&q.k2);
                 const f2 C1 = bc2(v0.x), D2 = bc2(v0.y), D3 = bc2(v0.z), D4 = bc2(v0.w);
                 const f2 BT = bc2(v1.x), BP = bc2(v1.w), PY = bc2(v2.y);
-                const f2 XAP = bc2(xc * v1.z);
+                const f2 AP = bc2(v1.z);
                 const f2 PHX = bc2(fmaf(2.f * xc, v2.x, v1.y));
 #pragma unroll
                 for (int h = 0; h < kPix / 2; ++h) {
                     const f2 qc = fmul2(QQ2[h], C1);
-                    const f2 m = ffma2(YC2[h], BP, fadd2(XAP, qc));
+                    const f2 m = ffma2(YC2[h], BP, ffma2(XC2, AP, qc));
                     const f2 m2 = fmul2(m, m);
                     const f2 poly = NTERMS == 4 ? ffma2(m, ffma2(m, D4, D3), D2) : ffma2(m, D3, D2);
                     const f2 dR = ffma2(m2, poly, m);
@@ -821,10 +851,12 @@ __global__ void __launch_bounds__(kThreads, SARBP_BP_MINBLOCKS)
                 const float4 v0 = lds128(smem_addr(&q.k0)), v1 = lds128(smem_addr(&q.k1));
                 const f2 C1 = bc2(v0.x), C2 = bc2(v0.y), C3 = bc2(v0.z), C4 = bc2(v0.w);
                 const f2 BT = bc2(v1.x), PHT = bc2(v1.y), BB = bc2(v1.w);
-                const f2 XA = bc2(xc * v1.z);
+                const f2 AA = bc2(v1.z);
 #pragma unroll
                 for (int h = 0; h < kPix / 2; ++h) {
-                    const f2 n = ffma2(YC2[h], BB, fadd2(XA, QQ2[h]));
+                    // x A + |q|^2 in one rounding, as the projection's mul + add
+                    // compiles: the phase of a pixel depends on it in the last bits
+                    const f2 n = ffma2(YC2[h], BB, ffma2(XC2, AA, QQ2[h]));
                     f2 poly = NTERMS == 4 ? ffma2(n, ffma2(n, C4, C3), C2) : ffma2(n, C3, C2);
                     poly = ffma2(n, poly, C1);
                     const f2 dR = fmul2(n, poly);
@@ -920,6 +952,8 @@ __global__ void __launch_bounds__(kThreads, SARBP_BP_MINBLOCKS)
                 }
             }
         }
+        }
+        if constexpr (kHelpers) failed = __syncthreads_or(failed);
     }
 
     if (CHECKED && clamped) atomicOr(P.err, kErrIndexClamp);
@@ -931,13 +965,15 @@ __global__ void __launch_bounds__(kThreads, SARBP_BP_MINBLOCKS)
 
     if constexpr (ADJ) {
         if (nchunks > 0) {
-            __syncthreads();
+            if (!kHelpers) __syncthreads();
             const int last = nchunks - 1;
-            flush_projection(P, S, last & 1, p_begin + last * chunk, min(chunk, p_end - p_begin - last * chunk));
+            if (warp == kStager0)
+                flush_projection(P, S, last & 1, p_begin + last * chunk, min(chunk, p_end - p_begin - last * chunk), lane);
         }
         return;
     }
 
+    if (helper) return;
     if constexpr (kSplitBp) {  // s e^{j phase}: (s.x cos - s.y sin, s.y cos + s.x sin)
 #pragma unroll
         for (int j = 0; j < kPix; ++j) {
@@ -990,13 +1026,14 @@ template <int MODE, int STORE, int NTERMS, bool CHECKED, int PIX, bool ADJ = fal
           bool LIN = false>
 cudaError_t launch_variant(const BpPlan &p, cudaStream_t s, int tiles, int tiles_y, int pps, float qq_max) {
     if (CHUNK && p.chunk != CHUNK) return cudaErrorInvalidValue;
+    constexpr int threads = kThreads + 32 * helper_warps<MODE, CHECKED, PIX, ADJ, CHUNK, LIN>();
     auto k = bp_kernel<MODE, STORE, NTERMS, CHECKED, PIX, ADJ, CHUNK, TESTF, LIN>;
     const size_t smem = bp_smem_bytes(STORE, p.win, p.chunk);
     cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void *>(k));
     if (e != cudaSuccess) return e;
-    if (t_occupancy) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(t_occupancy, k, kThreads, smem);
+    if (t_occupancy) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(t_occupancy, k, threads, smem);
     dim3 grid(tiles, p.segments);
-    k<<<grid, kThreads, smem, s>>>(p, tiles_y, pps, qq_max);
+    k<<<grid, threads, smem, s>>>(p, tiles_y, pps, qq_max);
     return cudaGetLastError();
 }
 
