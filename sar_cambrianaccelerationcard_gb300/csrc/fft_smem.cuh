@@ -18,6 +18,9 @@ namespace {
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
     return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
 }
+__device__ __forceinline__ float2 cfma(float2 a, float2 b, float2 c) {  // a b + c
+    return make_float2(fmaf(a.x, b.x, fmaf(-a.y, b.y, c.x)), fmaf(a.x, b.y, fmaf(a.y, b.x, c.y)));
+}
 // Complex add / subtract as one packed FP32x2 instruction (sm_100+ f32x2:
 // each half rounded to nearest, the same results as two scalar operations):
 // a float2 already lives in a register pair, so the butterflies' add network
@@ -67,24 +70,29 @@ __device__ __forceinline__ float2 mulj(float2 a) {
 // the stride-16 stores of the first radix-16 stage.  The swizzle only changes
 // bits 0..3 and depends on bits 4..7, so sw(x + c) = sw(x) + c for any
 // multiple c of 256.
-__host__ __device__ constexpr int sw(int x) { return x ^ (((x >> 4) & 15) ^ ((x >> 3) & 8)); }
-
-// table slot of entry i: one spare slot per 8 entries, so strided gathers
-// spread over the banks
-__device__ __forceinline__ int tslot(int i) { return i + (i >> 3); }
+// Transforms that start with a radix-32 stage take t = (x >> 5) & 15 alone: their
+// first stores run at stride 32, which the form above hits twice per bank pair
+// (shared wavefronts of a 16384-point inverse -19%, range compression of 4096
+// pulses 2.74 -> 2.58 ms, 8192 points -5%), and their other accesses are contiguous
+// runs.  It depends on bits 5..8, so there sw(x + c) = sw(x) + c for multiples c
+// of 512.
+template <bool R32>
+__host__ __device__ constexpr int sw_t(int x) {
+    return R32 ? x ^ ((x >> 5) & 15) : x ^ (((x >> 4) & 15) ^ ((x >> 3) & 8));
+}
 
 constexpr int kWlo = 128;  // low level of the transform twiddle table
 
-// Shared-memory tables.  E^m = e^{+j 2 pi m / (L N)} (upsampling ramp, split
-// combine) from E^m = T_hi[m >> 8] * T_lo[m & 255]; the transform twiddles
-// W^m = e^{+j 2 pi m / N} = E^{L m} from W^m = W_hi[m >> 7] * W_lo[m & 127].
+// E^m = e^{+j 2 pi m / (L N)} (upsampling ramp, split combine) from the two-level
+// table in global memory, E^m = T[256 + (m >> 8)] * T[m & 255]; the transform
+// twiddles W^m = e^{+j 2 pi m / N} = E^{L m} from a second two-level table in
+// shared memory, W^m = W_hi[m >> 7] * W_lo[m & 127].
 struct Etab {
-    const float2 *lo;   // E^i, i < 256 (or L N entries when L N < 256), slot tslot(i)
-    const float2 *hi;   // E^{256 i}, i < max(1, L N / 256), slot tslot(i)
+    const float2 *e;    // E^i, i < 256, then E^{256 i}, i < max(1, L N / 256)
     const float2 *wlo;  // W^i, i < min(N, 128)
     const float2 *whi;  // W^{128 i}, i < max(1, N / 128)
     __device__ __forceinline__ float2 operator()(int m) const {
-        return cmul(hi[tslot(m >> 8)], lo[tslot(m & 255)]);
+        return cmul(__ldg(&e[256 + (m >> 8)]), __ldg(&e[m & 255]));
     }
     __device__ __forceinline__ float2 w(int m) const { return cmul(whi[m >> 7], wlo[m & (kWlo - 1)]); }
 };
@@ -335,6 +343,36 @@ __device__ __forceinline__ void twiddles(const Etab &E, int m, float2 lo1, float
     }
 }
 
+#ifndef SARBP_FFT_RADIX16
+#define SARBP_FFT_RADIX16 1
+#endif
+// radix-32 stages where every thread holds at least one 32-point butterfly
+// (N / 32 >= T: transforms with at least 32 points per thread): two
+// shared-memory passes instead of three for 16384 points at 512 threads
+// (32-32-16) and 8192 at 256 (32-32-8).  Range compression on GB300, 4096
+// pulses: 16384 points 3.077 -> 2.986 ms, 8192 points 1.295 -> 1.123 ms; 32768
+// (2048 pulses) 4.289 -> 4.170 ms.  Shapes with fewer points per thread (the
+// omega-K transforms) keep their radix-16/8 stages.
+#ifndef SARBP_FFT_RADIX32
+#define SARBP_FFT_RADIX32 1
+#endif
+// Radix of the stage with stride Ns (the same sequence as Stages).
+template <int N, int T, int Ns>
+__host__ __device__ constexpr int stage_radix() {
+    return (SARBP_FFT_RADIX32 && Ns * 32 <= N && N / 32 >= T)   ? 32
+           : (SARBP_FFT_RADIX16 && Ns * 16 <= N && N / 16 >= T) ? 16
+           : (Ns * 8 <= N ? 8 : N / Ns);
+}
+
+template <int N, int T>
+__host__ __device__ constexpr int sw(int x) {
+    return sw_t<stage_radix<N, T, 1>() == 32>(x);
+}
+template <int N, int T>
+__host__ __device__ constexpr int sw_period() {
+    return stage_radix<N, T, 1>() == 32 ? 512 : 256;
+}
+
 // One Stockham stage: butterfly j reads s[j + r*N/R], applies twiddles
 // W_N^{k r N/(Ns R)} (k = j mod Ns), runs a radix-R DFT and writes
 // s[(j - k) R + k + r Ns] (slots through sw()).  Ns is a compile-time
@@ -349,8 +387,19 @@ struct SmemSink {};
 // BATCH > 1: the stage runs over BATCH independent N-point arrays CS points
 // apart (s + c CS), their butterflies spread over the threads and sharing the
 // stage's barriers.
-template <int N, int R, int T, bool INV, int Ns, class Sink = SmemSink, int BATCH = 1, int CS = N>
-__device__ __forceinline__ void stage(float2 *s, const Etab &E, Sink sink = Sink{}) {
+// tid, bar: this thread's place among the transform's T threads and their barrier
+// (the whole block, or one group of it).
+struct BlockBar {
+    __device__ __forceinline__ void sync() const { __syncthreads(); }
+};
+template <int T>
+struct GroupBar {
+    int id;  // named barrier
+    __device__ __forceinline__ void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(T) : "memory"); }
+};
+template <int N, int R, int T, bool INV, int Ns, class Sink = SmemSink, int BATCH = 1, int CS = N, class Bar = BlockBar>
+__device__ __forceinline__ void stage(float2 *s, const Etab &E, Sink sink = Sink{}, int tid = threadIdx.x,
+                                      Bar bar = Bar{}) {
     constexpr bool kToSmem = std::is_same<Sink, SmemSink>::value;
     constexpr int NB = N / R;
     constexpr int NBT = NB * BATCH;
@@ -360,22 +409,29 @@ __device__ __forceinline__ void stage(float2 *s, const Etab &E, Sink sink = Sink
     float2 v[PER][R];
 #pragma unroll
     for (int b = 0; b < PER; ++b) {
-        const int jj = threadIdx.x + b * T;
+        const int jj = tid + b * T;
         if (PER * T == NBT || jj < NBT) {
             const int col = BATCH == 1 ? 0 : jj / NB;
             const int j = jj - col * NB;
             const float2 *sc = s + col * CS;
-            if constexpr (NB % 256 == 0) {
-                const float2 *src = sc + sw(j);
+            constexpr int P = sw_period<N, T>();
+            if constexpr (NB % P == 0) {
+                const float2 *src = sc + sw<N, T>(j);
 #pragma unroll
                 for (int r = 0; r < R; ++r) v[b][r] = src[r * NB];
+            } else if constexpr (2 * NB % P == 0 && R % 2 == 0) {
+                const float2 *even = sc + sw<N, T>(j), *odd = sc + sw<N, T>(j + NB);
+#pragma unroll
+                for (int r = 0; r < R; r += 2) {
+                    v[b][r] = even[r * NB];
+                    v[b][r + 1] = odd[r * NB];
+                }
             } else {
 #pragma unroll
-                for (int r = 0; r < R; ++r) v[b][r] = sc[sw(j + r * NB)];
+                for (int r = 0; r < R; ++r) v[b][r] = sc[sw<N, T>(j + r * NB)];
             }
         }
     }
-    if constexpr (kToSmem) __syncthreads();  // loads done before the in-place stores
     float2 w[R <= 8 ? R : 1];
     Tw16 t16;
     Tw32 t32;
@@ -388,13 +444,13 @@ __device__ __forceinline__ void stage(float2 *s, const Etab &E, Sink sink = Sink
     float2 lo[5] = {lo1, lo1, lo1, lo1, lo1};
     if constexpr (kSameK) {
         if constexpr (R == 32)
-            t32 = tw32_bases<INV, false>(E, C * (int)(threadIdx.x & (Ns - 1)), lo);
+            t32 = tw32_bases<INV, false>(E, C * (tid & (Ns - 1)), lo);
         else if constexpr (R == 16)
-            t16 = tw16_bases<INV, false>(E, C * (int)(threadIdx.x & (Ns - 1)), lo);
+            t16 = tw16_bases<INV, false>(E, C * (tid & (Ns - 1)), lo);
         else
-            twiddles<R, INV, false>(E, C * (int)(threadIdx.x & (Ns - 1)), lo1, lo2, lo4, w);
+            twiddles<R, INV, false>(E, C * (tid & (Ns - 1)), lo1, lo2, lo4, w);
     } else if constexpr (kHoistLo) {
-        const int m = C * (int)threadIdx.x;
+        const int m = C * tid;
         lo1 = E.wlo[m & (kWlo - 1)];
         if (R >= 4) lo2 = E.wlo[(2 * m) & (kWlo - 1)];
         if (R >= 8) lo4 = E.wlo[(4 * m) & (kWlo - 1)];
@@ -408,11 +464,10 @@ __device__ __forceinline__ void stage(float2 *s, const Etab &E, Sink sink = Sink
     }
 #pragma unroll
     for (int b = 0; b < PER; ++b) {
-        const int jj = threadIdx.x + b * T;
+        const int jj = tid + b * T;
         if (PER * T == NBT || jj < NBT) {
             const int col = BATCH == 1 ? 0 : jj / NB;
             const int j = jj - col * NB;
-            float2 *sc = s + col * CS;
             const int k = j & (Ns - 1);
             if constexpr (Ns > 1) {
                 if constexpr (R == 32) {
@@ -428,36 +483,41 @@ __device__ __forceinline__ void stage(float2 *s, const Etab &E, Sink sink = Sink
                 }
             }
             Dft<R, INV>::run(v[b]);
-            const int x0 = (j - k) * R + k;
             if constexpr (!kToSmem) {
+                const int x0 = (j - k) * R + k;
 #pragma unroll
                 for (int r = 0; r < R; ++r) sink(x0 + r * Ns, v[b][r]);
-            } else if constexpr (Ns % 256 == 0) {
-                float2 *dst = sc + sw(x0);
-#pragma unroll
-                for (int r = 0; r < R; ++r) dst[r * Ns] = v[b][r];
-            } else {
-#pragma unroll
-                for (int r = 0; r < R; ++r) sc[sw(x0 + r * Ns)] = v[b][r];
             }
         }
     }
-    if constexpr (kToSmem) __syncthreads();
+    if constexpr (kToSmem) {
+        // every thread's loads before the in-place stores.  After the butterflies,
+        // not before them: a warp computes as soon as its own points have arrived
+        // (config-2 range compression 2.91 -> 2.84 ms, omega-K 834 -> 816 us)
+        bar.sync();
+#pragma unroll
+        for (int b = 0; b < PER; ++b) {
+            const int jj = tid + b * T;
+            if (PER * T == NBT || jj < NBT) {
+                const int col = BATCH == 1 ? 0 : jj / NB;
+                const int j = jj - col * NB;
+                float2 *sc = s + col * CS;
+                const int k = j & (Ns - 1);
+                const int x0 = (j - k) * R + k;
+                if constexpr (Ns % sw_period<N, T>() == 0) {
+                    float2 *dst = sc + sw<N, T>(x0);
+#pragma unroll
+                    for (int r = 0; r < R; ++r) dst[r * Ns] = v[b][r];
+                } else {
+#pragma unroll
+                    for (int r = 0; r < R; ++r) sc[sw<N, T>(x0 + r * Ns)] = v[b][r];
+                }
+            }
+        }
+        bar.sync();
+    }
 }
 
-#ifndef SARBP_FFT_RADIX16
-#define SARBP_FFT_RADIX16 1
-#endif
-// radix-32 stages where every thread holds at least one 32-point butterfly
-// (N / 32 >= T: transforms with at least 32 points per thread): two
-// shared-memory passes instead of three for 16384 points at 512 threads
-// (32-32-16) and 8192 at 256 (32-32-8).  Range compression on GB300, 4096
-// pulses: 16384 points 3.077 -> 2.986 ms, 8192 points 1.295 -> 1.123 ms; 32768
-// (2048 pulses) 4.289 -> 4.170 ms.  Shapes with fewer points per thread (the
-// omega-K transforms) keep their radix-16/8 stages.
-#ifndef SARBP_FFT_RADIX32
-#define SARBP_FFT_RADIX32 1
-#endif
 // radix-16 stages while 16 * Ns <= N and the stage keeps all T threads busy
 // (N / 16 >= T), then radix-8 stages while 8 * Ns <= N, then one radix-4 or
 // radix-2 stage
@@ -489,14 +549,13 @@ __device__ void fft_smem(float2 *s, const Etab &E) {
 }
 
 // BATCH transforms of N points, array c at s + c CS, sharing each stage's
-// barriers (same radix sequence as Stages).
+// barriers: radix-16 stages while the batch's butterflies keep all T threads
+// busy (4 x 4096 points at 512 threads: 16-16-16 instead of 8-8-8-8, omega-K image
+// 799 -> 791 us), then as Stages.
 template <int N, int T, bool INV, int Ns, int BATCH, int CS>
 struct StagesBatched {
     __device__ __forceinline__ static void run(float2 *s, const Etab &E) {
-        if constexpr (SARBP_FFT_RADIX32 && Ns * 32 <= N && N / 32 >= T) {
-            stage<N, 32, T, INV, Ns, SmemSink, BATCH, CS>(s, E);
-            StagesBatched<N, T, INV, Ns * 32, BATCH, CS>::run(s, E);
-        } else if constexpr (SARBP_FFT_RADIX16 && Ns * 16 <= N && N / 16 >= T) {
+        if constexpr (Ns * 16 <= N && N * BATCH / 16 >= T) {
             stage<N, 16, T, INV, Ns, SmemSink, BATCH, CS>(s, E);
             StagesBatched<N, T, INV, Ns * 16, BATCH, CS>::run(s, E);
         } else if constexpr (Ns * 8 <= N) {
@@ -509,14 +568,6 @@ struct StagesBatched {
         }
     }
 };
-
-// Radix of the stage with stride Ns (the same sequence as Stages).
-template <int N, int T, int Ns>
-__host__ __device__ constexpr int stage_radix() {
-    return (SARBP_FFT_RADIX32 && Ns * 32 <= N && N / 32 >= T)   ? 32
-           : (SARBP_FFT_RADIX16 && Ns * 16 <= N && N / 16 >= T) ? 16
-           : (Ns * 8 <= N ? 8 : N / Ns);
-}
 
 // I/O-fused transform.  The first stage (stride 1) takes its inputs from
 // registers: butterfly j = threadIdx.x + b T (j < N / R) holds points
@@ -533,8 +584,8 @@ struct FirstIn {
     static constexpr int NB = N / R;
     static constexpr int PER = (NB + T - 1) / T;
     static_assert(R < N, "I/O-fused transforms need at least two stages");
-    __device__ __forceinline__ static bool live(int b) { return PER * T == NB || (int)threadIdx.x + b * T < NB; }
-    __device__ __forceinline__ static int point(int b, int r) { return (int)threadIdx.x + b * T + r * NB; }
+    __device__ __forceinline__ static bool live(int b, int tid = threadIdx.x) { return PER * T == NB || tid + b * T < NB; }
+    __device__ __forceinline__ static int point(int b, int r, int tid = threadIdx.x) { return tid + b * T + r * NB; }
 };
 
 template <int N, int T, bool INV, int Ns, class Sink>
@@ -560,46 +611,83 @@ __device__ __forceinline__ void fft_io(float2 *s, const Etab &E, float2 (&v)[Fir
             const int j = (int)threadIdx.x + b * T;
             Dft<R, INV>::run(v[b]);
 #pragma unroll
-            for (int r = 0; r < R; ++r) s[sw(j * R + r)] = v[b][r];  // stride 1: x0 = j R
+            for (int r = 0; r < R; ++r) s[sw<N, T>(j * R + r)] = v[b][r];  // stride 1: x0 = j R
         }
     }
     __syncthreads();
     StagesTo<N, T, INV, R, Sink>::run(s, E, sink);
 }
 
-// Shared memory after the N points: E low/high levels (slots through
-// tslot), W low/high levels, and the per-CTA ramp table of the inverse.
-constexpr int kEloSlots = 288, kEhiSlots = 1152, kWhiMax = 128, kRampMax = 64;
-constexpr size_t kTabSmem = sizeof(float2) * (kEloSlots + kEhiSlots + kWlo + kWhiMax + kRampMax);
-template <int N>
-__device__ __forceinline__ float2 *ramp_slots(float2 *sm) {
-    return sm + N + kEloSlots + kEhiSlots + kWlo + kWhiMax;
+// G transforms by a block of G T threads, group g = threadIdx.x / T holding the
+// first-stage points of array g (s + g CS).  The groups run their stages on their
+// own barriers; in the last one the block's threads take the butterflies with
+// the array index fastest, so sink(g, x, value) runs on neighbouring lanes for
+// the G arrays' same output point.
+template <int N, int T, bool INV, int Ns, int G, int CS, class Sink>
+struct StagesGroup {
+    __device__ __forceinline__ static void run(float2 *s, const Etab &E, Sink sink) {
+        constexpr int R = stage_radix<N, T, Ns>();
+        const int group = threadIdx.x / T;
+        if constexpr (Ns * R == N) {
+            __syncthreads();
+            const int g = threadIdx.x % G;
+            auto one = [&](int x, float2 v) { sink(g, x, v); };
+            stage<N, R, T, INV, Ns, decltype(one), 1, N, BlockBar>(s + g * CS, E, one, threadIdx.x / G);
+        } else {
+            stage<N, R, T, INV, Ns, SmemSink, 1, N, GroupBar<T>>(s + group * CS, E, SmemSink{}, threadIdx.x % T,
+                                                              GroupBar<T>{1 + group});
+            StagesGroup<N, T, INV, Ns * R, G, CS, Sink>::run(s, E, sink);
+        }
+    }
+};
+template <int N, int T, bool INV, int G, int CS, class Sink>
+__device__ __forceinline__ void fft_io_group(float2 *s, const Etab &E,
+                                             float2 (&v)[FirstIn<N, T>::PER][FirstIn<N, T>::R], Sink sink) {
+    using F = FirstIn<N, T>;
+    constexpr int R = F::R;
+    const int group = threadIdx.x / T, tid = threadIdx.x % T;
+    float2 *sg = s + group * CS;
+#pragma unroll
+    for (int b = 0; b < F::PER; ++b) {
+        if (F::live(b, tid)) {
+            const int j = tid + b * T;
+            Dft<R, INV>::run(v[b]);
+#pragma unroll
+            for (int r = 0; r < R; ++r) sg[sw<N, T>(j * R + r)] = v[b][r];  // stride 1: x0 = j R
+        }
+    }
+    __syncthreads();  // also publishes the block's W tables
+    StagesGroup<N, T, INV, R, G, CS, Sink>::run(s, E, sink);
 }
 
-// Fills the E tables from global memory, then derives the W tables
-// (W^m = E^{L m}).  Contains one block barrier; the caller synchronises again
-// before the W tables are read.
-template <int N, int T>
+// Shared memory after the points: W low/high levels and the per-CTA ramp table
+// of the inverse range transform.
+constexpr int kWhiMax = 128, kRampMax = 64;
+constexpr size_t kTabSmem = sizeof(float2) * (kWlo + kWhiMax + kRampMax);
+template <int N>
+__device__ __forceinline__ float2 *ramp_slots(float2 *sm) {
+    return sm + N + kWlo + kWhiMax;
+}
+
+// Fills the W tables (W^m = E^{L m}) straight from the global E table, which the
+// CTAs of an SM share in L1: no barrier here (the caller synchronises before the
+// W tables are read).  Copying the E table to shared memory first cost up to
+// 18 KB per CTA, a barrier before the W tables could be derived and 15% of the
+// shared wavefronts: range compression of 4096 16384-point pulses 2.84 -> 2.74 ms,
+// 8192 points -4%, omega-K image 816 -> 799 us.
+template <int N, int T, int BLOCK = T>
 __device__ __forceinline__ Etab load_etab_at(float2 *tables, const float2 *__restrict__ etab, int L) {
     static_assert(N / kWlo <= kWhiMax, "W table too small");
-    const int LN = L * N;
-    const int nlo = LN < 256 ? LN : 256;
-    const int nhi = LN < 256 ? 1 : LN / 256;
-    float2 *lo = tables;
-    float2 *hi = lo + kEloSlots;
-    float2 *wlo = hi + kEhiSlots;
+    float2 *wlo = tables;
     float2 *whi = wlo + kWlo;
-    for (int i = threadIdx.x; i < nlo; i += T) lo[tslot(i)] = __ldg(&etab[i]);
-    for (int i = threadIdx.x; i < nhi; i += T) hi[tslot(i)] = __ldg(&etab[256 + i]);
-    __syncthreads();
-    const Etab E{lo, hi, wlo, whi};
+    const Etab E{etab, wlo, whi};
     constexpr int nwlo = N < kWlo ? N : kWlo;
     constexpr int nwhi = N < kWlo ? 1 : N / kWlo;
-    for (int i = threadIdx.x; i < nwlo + nwhi; i += T) {
+    for (int i = threadIdx.x; i < nwlo + nwhi; i += BLOCK) {
         if (i < nwlo)
             wlo[i] = E(L * i);
         else
-            whi[i - nwlo] = E((L * kWlo * (i - nwlo)) & (LN - 1));
+            whi[i - nwlo] = E((L * kWlo * (i - nwlo)) & (L * N - 1));
     }
     return E;
 }
@@ -610,11 +698,14 @@ __device__ __forceinline__ Etab load_etab(float2 *sm, const float2 *__restrict__
 }
 
 // CTAs per SM that a T-thread kernel holding an N-point transform (plus the
-// tables) aims its register allocation at: two when both fit twice (8192
-// points at 512 threads: 64 registers per thread), else one.
+// tables) aims its register allocation at: what fits 227 KB of shared memory and
+// 65536 registers at 128 per thread (32 points per thread) or 64 (fewer).
 template <int N, int T>
-constexpr int fft_min_blocks() {
-    return (T * 64 <= 32768 && (size_t)N * 8 + kTabSmem <= (size_t)110 * 1024) ? 2 : 1;
+__host__ __device__ constexpr int fft_min_blocks() {
+    const int by_smem = (int)((227u << 10) / (sizeof(float2) * N + kTabSmem + 1024));
+    const int by_regs = 65536 / (T * (N / T >= 32 ? 128 : 64));
+    const int n = by_smem < by_regs ? by_smem : by_regs;
+    return n < 1 ? 1 : n > 16 ? 16 : n;
 }
 
 }  // namespace

@@ -9,30 +9,38 @@
 //               G[k] = conj(H[k]) e^{-j2pi k D/N} / N -> spectrum scratch.
 //               Also emits the per-pulse bound sum_k |Y[k]| (>= max |output|)
 //               from which the FP16 storage scale is derived.
-//   rc_inverse  (one CTA per pulse and upsampling phase r): the L*N-point
+//   rc_inverse  (one or two upsampling phases r per CTA): the L*N-point
 //               inverse of the zero-inserted spectrum evaluated at bins
 //               b = L*i + r equals the N-point inverse of Y[k]*e^{+j2pi kappa r/(LN)}
-//               (kappa = signed frequency), so each CTA runs one N-point
-//               inverse FFT and writes every L-th output bin.
+//               (kappa = signed frequency), so a phase is one N-point inverse
+//               FFT whose outputs are every L-th bin of the row.
 //
 // The FFT is a Stockham autosort transform with radix-32/16/8 stages (one
 // radix-4 or radix-2 stage for the remaining factor), in place in shared
 // memory (XOR-swizzled so every stage's accesses are free of bank conflicts)
 // with a barrier between each stage's loads and stores.  The upsampling ramp
-// is a power of E = e^{j 2 pi / (L N)}, read from a two-level table in shared
-// memory, E^m = T_hi[m >> 8] * T_lo[m & 255] (computed in double precision on
-// the host); the transform twiddles are powers of W = E^L from a second
-// two-level table derived from it at kernel start, so no FFT stage touches
+// is a power of E = e^{j 2 pi / (L N)}, from a two-level table in global memory,
+// E^m = T_hi[m >> 8] * T_lo[m & 255] (computed in double precision on the host);
+// the transform twiddles are powers of W = E^L from a second two-level table
+// derived from it into shared memory at kernel start, so no FFT stage touches
 // global memory.
 //
 // N = 32768 (shared memory holds 16384 points) is split by one radix-2 stage:
 // the forward runs two CTAs per pulse on the half-size inputs x[n] + x[n+M] and
-// (x[n] - x[n+M]) W_N^n, giving the even and odd spectral bins; the inverse
-// runs a 2-CTA cluster per (pulse, phase) on the even and odd bins and forms
-// y[i] = A[i] + W_N^{-i} B[i], y[i+M] = A[i] - W_N^{-i} B[i] with the partner's
-// half read through distributed shared memory.
-#include <cooperative_groups.h>
-
+// (x[n] - x[n+M]) W_N^n, giving the even and odd spectral bins; the inverse folds
+// the ramped spectrum modulo M = 16384 while loading it, Y[k] E^{kappa r} +
+// Y[k+M] E^{kappa' r} for r < 2 L, which is upsampling by 2 L of an M-point
+// transform and needs no exchange between CTAs.  (A 2-CTA cluster per phase that
+// combined its halves through distributed shared memory: 768 pulses 1.61 ms,
+// folded 1.30, 1.23 with the table and layout changes of fft_smem.cuh.)  Folding
+// smaller transforms does not pay: 16384 points as 2 x 8192, two CTAs per SM,
+// 3.39 against 2.87 ms for 4096 pulses, for a store then touches 32 lines and
+// every fold adds a complex product per point.
+//
+// What bounds the inverse: the load/store path (shared wavefronts of the two
+// passes, 48% of them at 8192 points the strided stores; 74% busy there) and, at
+// 16384 points, that one 131 KB CTA per SM runs its load, butterfly and store
+// phases one after the other.
 #include "fft_smem.cuh"
 
 namespace sarbp {
@@ -52,6 +60,12 @@ __device__ __forceinline__ float block_sum(float v, float *red) {
         for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
     }
     return t;  // valid in thread 0
+}
+
+// The FP16 storage scale from the bound on |output|: a power of two, so that
+// stored magnitudes stay <= 2^14.
+__device__ __forceinline__ float storage_scale(float bound) {
+    return bound > 0.f && isfinite(bound) ? exp2f(ceilf(log2f(bound) - 14.f)) : 1.f;
 }
 
 // SCALE: also the per-pulse bound sum_k |Y[k]| and the FP16 storage scale
@@ -87,50 +101,57 @@ __global__ void __launch_bounds__(T, (fft_min_blocks<N, T>())) rc_forward_kernel
     });
     if constexpr (!SCALE) return;
     const float bound = block_sum<T>(acc, red);
-    if (threadIdx.x == 0) {
-        // power-of-two scale so that stored FP16 magnitudes stay <= 2^14
-        float sc = 1.f;
-        if (bound > 0.f && isfinite(bound)) sc = exp2f(ceilf(log2f(bound) - 14.f));
-        scale[p] = sc;
-    }
+    if (threadIdx.x == 0) scale[p] = storage_scale(bound);
 }
 
-template <int N, int T, int STORE>
-__global__ void __launch_bounds__(T, (fft_min_blocks<N, T>())) rc_inverse_kernel(int ns, int L, int nbins,
-                                                       const float2 *__restrict__ spec,
-                                                       const float2 *__restrict__ etab,
-                                                       const float *__restrict__ scale,
-                                                       void *__restrict__ out) {
+// N-bin spectrum, M-point transforms (M divides N), G of them per CTA: CTA (p, r0)
+// gives the bins (L N / M) i + r of the phases r = G r0 .. G r0 + G - 1, r < L N / M,
+// each the M-point inverse of the spectrum times its ramp folded modulo M.  The
+// G phases' bins are neighbours in the row, and the last stage's lanes store
+// them together.
+// points between the arrays: in the last stage a half-warp loads 16 / G points of
+// each, from disjoint banks
+template <int G>
+constexpr int group_pad = G > 1 ? 16 / G : 0;
+template <int N, int M, int T, int G, int STORE>
+__global__ void __launch_bounds__(G *T, (fft_min_blocks<G * M, G * T>()))
+    rc_inverse_kernel(int L, int nbins, const float2 *__restrict__ spec, const float2 *__restrict__ etab,
+                      const float *__restrict__ bound2, float *__restrict__ scale, void *__restrict__ out) {
     extern __shared__ float2 sm[];
-    const int p = blockIdx.x / L;
-    const int r = blockIdx.x - p * L;
+    constexpr int FOLD = N / M, CS = M + group_pad<G>;
+    const int LF = L * FOLD, per = LF / G;
+    const int group = G > 1 ? threadIdx.x / T : 0, tid = G > 1 ? threadIdx.x % T : threadIdx.x;
+    const int p = blockIdx.x / per;
+    const int r0 = (blockIdx.x - p * per) * G, r = r0 + group;
     const float2 *in = spec + (size_t)p * N;
     const int LN = L * N;
     // first-stage inputs straight from the spectrum, issued before the tables
-    using F = FirstIn<N, T>;
+    using F = FirstIn<M, T>;
     float2 v[F::PER][F::R];
 #pragma unroll
     for (int b = 0; b < F::PER; ++b)
 #pragma unroll
         for (int q = 0; q < F::R; ++q)
-            v[b][q] = F::live(b) ? __ldg(&in[F::point(b, q)]) : make_float2(0.f, 0.f);
-    const Etab E = load_etab<N, T>(sm, etab, L);
+            v[b][q] = F::live(b, tid) ? __ldg(&in[F::point(b, q, tid)]) : make_float2(0.f, 0.f);
+    float2 *tables = sm + G * CS;
+    const Etab E = load_etab_at<M, T, G * T>(tables, etab, LF);
     // Ramp E^{kappa r}, kappa the signed frequency (MATLAB split floor((N+1)/2)
     // = N/2 for even N).  With k = tid + T i (every first-stage point of a
-    // thread is congruent to tid mod T when N / R is a multiple of T) and N/2 a
-    // multiple of T it factors into a per-thread E^{tid r} and a per-CTA table
+    // thread is congruent to tid mod T when M / R is a multiple of T) and N/2 a
+    // multiple of T it factors into a per-thread E^{tid r} and a per-phase table
     // over i that also carries the E^{-N r} of the negative half.
     constexpr bool kTwoLevel = (N / 2) % T == 0 && N / T <= kRampMax && F::NB % T == 0;
-    float2 *rt = ramp_slots<N>(sm);
+    static_assert(kTwoLevel || FOLD == 1, "folded spectra use the two-level ramp");
+    float2 *rt = tables + kWlo + kWhiMax + group * kRampMax;
     float2 base = make_float2(1.f, 0.f);
     if (kTwoLevel && r != 0) {
-        if (threadIdx.x < N / T) {
-            const int i = threadIdx.x;
+        if (tid < N / T) {
+            const int i = tid;
             float2 w = E((T * i * r) & (LN - 1));
             if (T * i >= N / 2) w = cmul(w, E((LN - N * r) & (LN - 1)));
             rt[i] = w;
         }
-        base = E((int)(threadIdx.x * r) & (LN - 1));
+        base = E((tid * r) & (LN - 1));
     }
     __syncthreads();
     if (r != 0) {
@@ -138,30 +159,66 @@ __global__ void __launch_bounds__(T, (fft_min_blocks<N, T>())) rc_inverse_kernel
         for (int b = 0; b < F::PER; ++b)
 #pragma unroll
             for (int q = 0; q < F::R; ++q) {
-                const int k = F::point(b, q);
+                const int k = F::point(b, q, tid);
                 if (kTwoLevel) {
-                    v[b][q] = cmul(cmul(v[b][q], base), rt[k / T]);
+                    v[b][q] = cmul(v[b][q], rt[k / T]);
                 } else {
                     const int kap = k < N / 2 ? k : k - N;
                     v[b][q] = cmul(v[b][q], E((kap * r) & (LN - 1)));  // LN is a power of two
                 }
             }
+#pragma unroll
+        for (int f = 1; f < FOLD; ++f)
+#pragma unroll
+            for (int b = 0; b < F::PER; ++b)
+#pragma unroll
+                for (int q = 0; q < F::R; ++q) {
+                    const int k = F::point(b, q, tid) + f * M;
+                    v[b][q] = cfma(__ldg(&in[k]), rt[k / T], v[b][q]);
+                }
+        if (kTwoLevel) {
+#pragma unroll
+            for (int b = 0; b < F::PER; ++b)
+#pragma unroll
+                for (int q = 0; q < F::R; ++q) v[b][q] = cmul(v[b][q], base);
+        }
+    } else {
+#pragma unroll
+        for (int f = 1; f < FOLD; ++f)
+#pragma unroll
+            for (int b = 0; b < F::PER; ++b)
+#pragma unroll
+                for (int q = 0; q < F::R; ++q) v[b][q] = cadd(v[b][q], __ldg(&in[F::point(b, q, tid) + f * M]));
     }
+    // outputs x of phase r0 + g: bin LF x + r0 + g, inside the row for x < live
+    const int last = r0 + (G > 1 ? (int)(threadIdx.x % G) : 0);
+    const int live = (nbins - last + LF - 1) / LF;
+    auto run = [&](auto store) {
+        if constexpr (G > 1)
+            fft_io_group<M, T, true, G, CS>(sm, E, v, [&](int, int x, float2 y) { store(x, y); });
+        else
+            fft_io<M, T, true>(sm, E, v, store);
+    };
     if (STORE == SARBP_STORE_C64) {
-        float2 *o = reinterpret_cast<float2 *>(out) + (size_t)p * nbins + r;
-        fft_io<N, T, true>(sm, E, v, [&](int i, float2 x) {
-            if (i < ns) o[(size_t)L * i] = x;
+        float2 *o = reinterpret_cast<float2 *>(out) + (size_t)p * nbins + last;
+        run([&](int x, float2 y) {
+            if (x < live) o[(size_t)LF * x] = y;
         });
     } else {
-        const float inv = 1.f / __ldg(&scale[p]);  // exact: scale is a power of two
-        __half2 *o = reinterpret_cast<__half2 *>(out) + (size_t)p * nbins + r;
-        fft_io<N, T, true>(sm, E, v, [&](int i, float2 x) {
-            if (i < ns) o[(size_t)L * i] = __floats2half2_rn(x.x * inv, x.y * inv);
+        float sc;
+        if (bound2) {  // the forward ran as two CTAs: combine their parts of the bound
+            sc = storage_scale(__ldg(&bound2[2 * p]) + __ldg(&bound2[2 * p + 1]));
+            if (r0 == 0 && threadIdx.x == 0) scale[p] = sc;
+        } else {
+            sc = scale[p];
+        }
+        const float inv = 1.f / sc;  // exact: scale is a power of two
+        __half2 *o = reinterpret_cast<__half2 *>(out) + (size_t)p * nbins + last;
+        run([&](int x, float2 y) {
+            if (x < live) o[(size_t)LF * x] = __floats2half2_rn(y.x * inv, y.y * inv);
         });
     }
 }
-
-namespace cg = cooperative_groups;
 
 // N = 2M forward: CTA pair (h = 0, 1) per pulse; h = 0 yields X[2k], h = 1 X[2k+1].
 // bound2[2p + h] receives the CTA's part of sum_k |Y[k]|.
@@ -204,75 +261,7 @@ __global__ void __launch_bounds__(T) rc_forward2_kernel(int ns, int L, const flo
     if (threadIdx.x == 0) bound2[2 * p + h] = bound;
 }
 
-// N = 2M inverse: cluster of two CTAs per (pulse, phase r).  CTA h transforms
-// the bins 2k + h, then each CTA writes half of the outputs using both halves.
-template <int M, int T, int STORE>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T)
-    rc_inverse2_kernel(int ns, int L, int nbins, const float2 *__restrict__ spec, const float2 *__restrict__ etab,
-                       const float *__restrict__ bound2, float *__restrict__ scale, void *__restrict__ out) {
-    extern __shared__ float2 sm[];
-    cg::cluster_group cluster = cg::this_cluster();
-    const int h = (int)cluster.block_rank();
-    const int pr = blockIdx.x >> 1;
-    const int p = pr / L, r = pr - p * L;
-    constexpr int N = 2 * M;
-    const int LN = L * N;
-    const float2 *in = spec + (size_t)p * N;
-    // first-stage inputs (bins 2k + h) straight into registers, issued before
-    // the table loads; the ramp needs the tables
-    using F = FirstIn<M, T>;
-    float2 v[F::PER][F::R];
-#pragma unroll
-    for (int b = 0; b < F::PER; ++b)
-#pragma unroll
-        for (int q = 0; q < F::R; ++q)
-            v[b][q] = F::live(b) ? __ldg(&in[2 * F::point(b, q) + h]) : make_float2(0.f, 0.f);
-    const Etab E = load_etab<M, T>(sm, etab, 2 * L);
-    if (r != 0) {  // the ramp reads only the E tables, published by load_etab's barrier
-#pragma unroll
-        for (int b = 0; b < F::PER; ++b)
-#pragma unroll
-            for (int q = 0; q < F::R; ++q) {
-                const int idx = 2 * F::point(b, q) + h;
-                const int kap = idx < N / 2 ? idx : idx - N;
-                v[b][q] = cmul(v[b][q], E((kap * r) & (LN - 1)));  // LN is a power of two
-            }
-    }
-    fft_io<M, T, true>(sm, E, v, SmemSink{});  // the partner reads the result from shared memory
-    cluster.sync();  // both halves transformed
-    const float2 *A = cluster.map_shared_rank(sm, 0);
-    const float2 *B = cluster.map_shared_rank(sm, 1);
-    float inv = 1.f;
-    if (STORE == SARBP_STORE_C32H) {
-        const float bound = __ldg(&bound2[2 * p]) + __ldg(&bound2[2 * p + 1]);
-        float sc = 1.f;
-        if (bound > 0.f && isfinite(bound)) sc = exp2f(ceilf(log2f(bound) - 14.f));
-        inv = 1.f / sc;
-        if (r == 0 && h == 0 && threadIdx.x == 0) scale[p] = sc;
-    }
-    const int i0 = h * (M / 2), i1 = i0 + M / 2;
-    for (int i = i0 + threadIdx.x; i < i1; i += T) {
-        const float2 a = A[sw(i)];
-        const float2 t = cmul(E(L * i), B[sw(i)]);  // W_N^{-i} B[i]
-        const float2 y0 = cadd(a, t), y1 = csub(a, t);
-        if (STORE == SARBP_STORE_C64) {
-            float2 *o = reinterpret_cast<float2 *>(out) + (size_t)p * nbins + r;
-            if (i < ns) o[(size_t)L * i] = y0;
-            if (i + M < ns) o[(size_t)L * (i + M)] = y1;
-        } else {
-            __half2 *o = reinterpret_cast<__half2 *>(out) + (size_t)p * nbins + r;
-            if (i < ns) o[(size_t)L * i] = __floats2half2_rn(y0.x * inv, y0.y * inv);
-            if (i + M < ns) o[(size_t)L * (i + M)] = __floats2half2_rn(y1.x * inv, y1.y * inv);
-        }
-    }
-    cluster.sync();  // the partner has finished reading this CTA's shared memory
-}
-
-// FFT sizes from this one up run as two half-size CTAs (forward) or 2-CTA
-// clusters (inverse); 32768 always does (its data exceed one CTA's shared memory).
-#ifndef SARBP_RC_SPLIT_MIN
-#define SARBP_RC_SPLIT_MIN 32768
-#endif
+constexpr int kInvPoints = 16384;  // largest inverse transform of one CTA
 // CTA sizes (threads) per transform length, measured on GB300 (ms for 4096
 // pulses, forward + eight inverse transforms each).  8192 points: 1.886 at
 // 1024 threads (one CTA per SM: its barriers are overlapped by nothing), 1.295
@@ -280,26 +269,24 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T)
 // radix-32 stages 32-32-8).  16384 points (128 KB, one CTA per SM whatever the
 // size): 3.077 at 1024 (16-16-16-4), 2.986 at 512 (32-32-16).  The 16384-point
 // halves of the 32768-point split path: 4.35 at 1024, 4.29 at 512 (radix-16),
-// 4.17 at 512 with radix-32 stages (2048 pulses).
-#ifndef SARBP_RC_8K_THREADS
-#define SARBP_RC_8K_THREADS 256
-#endif
-#ifndef SARBP_RC_BIG_THREADS
-#define SARBP_RC_BIG_THREADS 512
-#endif
-#ifndef SARBP_RC_HALF_THREADS
-#define SARBP_RC_HALF_THREADS 512
-#endif
+// 4.17 at 512 with radix-32 stages (2048 pulses).  4096 points: 16 per thread
+// (256 threads, 16-16-16) against 8 (512, 8-8-8-8): 512 pulses 95 -> 73 us.
 template <int N>
 constexpr int threads_for() {
-    return N >= 16384 ? SARBP_RC_BIG_THREADS : (N >= 8192 ? SARBP_RC_8K_THREADS : (N >= 4096 ? 512 : (N >= 512 ? N / 8 : 64)));
-}
-// the half-size transforms of the split path (two CTAs / a 2-CTA cluster per transform)
-template <int M>
-constexpr int threads_for_half() {
-    return M >= 16384 ? SARBP_RC_HALF_THREADS : threads_for<M>();
+    return N >= 16384 ? 512 : (N >= 2048 ? 256 : (N >= 512 ? N / 8 : 64));
 }
 
+// Phases per CTA of the inverse, measured (2048 pulses, L = 8, forward and
+// inverse, us at 1 / 2 / 4): 4096 points 301 / 246 / 254 (FP16 rows 270 / 261 / 262),
+// 8192 points 603 / 572 (FP16 rows 630 / 644), 2048 points 167 / 171 / 171.  A
+// phase's bins lie L bins apart, so a warp's store touches 16 lines of 128 bytes;
+// two phases' neighbouring bins halve that, which pays while the shared-memory and
+// store path bounds the kernel and the larger CTA costs no residency (two
+// 16384-point phases do not fit one SM).  Rows are divided evenly: L % G == 0.
+template <int N, int STORE>
+constexpr int phases_for() {
+    return N == 4096 || (N == 8192 && STORE == SARBP_STORE_C64) ? 2 : 1;
+}
 // With t_prepare set the launchers below configure their kernel and return
 // without launching it (prepare_rc_kernels).
 thread_local bool t_prepare = false;
@@ -317,55 +304,40 @@ cudaError_t fwd_n(const RcPlan &p, const float2 *echo, const float2 *filt, const
     return cudaGetLastError();
 }
 
-template <int N>
-cudaError_t inv_n(const RcPlan &p, const float2 *spec, const float2 *etab, const float *scale, void *out,
-                  cudaStream_t s) {
-    constexpr int T = threads_for<N>();
-    const size_t smem = sizeof(float2) * N + kTabSmem;
-    cudaError_t e;
-    if (p.storage == SARBP_STORE_C64) {
-        auto k = rc_inverse_kernel<N, T, SARBP_STORE_C64>;
-        e = allow_dynamic_smem(reinterpret_cast<const void *>(k));
-        if (e != cudaSuccess || t_prepare) return e;
-        k<<<p.np * p.L, T, smem, s>>>(p.ns, p.L, p.nbins, spec, etab, scale, out);
-    } else {
-        auto k = rc_inverse_kernel<N, T, SARBP_STORE_C32H>;
-        e = allow_dynamic_smem(reinterpret_cast<const void *>(k));
-        if (e != cudaSuccess || t_prepare) return e;
-        k<<<p.np * p.L, T, smem, s>>>(p.ns, p.L, p.nbins, spec, etab, scale, out);
-    }
+template <int N, int STORE, int G>
+cudaError_t inv_g(const RcPlan &p, const float2 *spec, const float2 *etab, const float *bound2, float *scale,
+                  void *out, cudaStream_t s) {
+    constexpr int M = N < kInvPoints ? N : kInvPoints, T = threads_for<M>();
+    const size_t smem = sizeof(float2) * (G * (M + group_pad<G>) + (G - 1) * kRampMax) + kTabSmem;
+    auto k = rc_inverse_kernel<N, M, T, G, STORE>;
+    cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void *>(k));
+    if (e != cudaSuccess || t_prepare) return e;
+    k<<<p.np * (p.L * (N / M) / G), G * T, smem, s>>>(p.L, p.nbins, spec, etab, bound2, scale, out);
     return cudaGetLastError();
+}
+template <int N, int STORE>
+cudaError_t inv_s(const RcPlan &p, const float2 *spec, const float2 *etab, const float *bound2, float *scale,
+                  void *out, cudaStream_t s) {
+    constexpr int G = phases_for<N, STORE>();
+    if (p.L % G == 0) return inv_g<N, STORE, G>(p, spec, etab, bound2, scale, out, s);
+    return inv_g<N, STORE, 1>(p, spec, etab, bound2, scale, out, s);
+}
+template <int N>
+cudaError_t inv_n(const RcPlan &p, const float2 *spec, const float2 *etab, const float *bound2, float *scale,
+                  void *out, cudaStream_t s) {
+    return p.storage == SARBP_STORE_C64 ? inv_s<N, SARBP_STORE_C64>(p, spec, etab, bound2, scale, out, s)
+                                        : inv_s<N, SARBP_STORE_C32H>(p, spec, etab, bound2, scale, out, s);
 }
 
 template <int M>
 cudaError_t fwd2(const RcPlan &p, const float2 *echo, const float2 *filt, const float2 *etab, float2 *spec,
                  float *bound2, cudaStream_t s) {
-    constexpr int T = threads_for_half<M>();
+    constexpr int T = threads_for<M>();
     const size_t smem = sizeof(float2) * M + kTabSmem;
     auto k = rc_forward2_kernel<M, T>;
     cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void *>(k));
     if (e != cudaSuccess || t_prepare) return e;
     k<<<2 * p.np, T, smem, s>>>(p.ns, p.L, echo, filt, etab, spec, bound2);
-    return cudaGetLastError();
-}
-
-template <int M>
-cudaError_t inv2(const RcPlan &p, const float2 *spec, const float2 *etab, const float *bound2, float *scale,
-                 void *out, cudaStream_t s) {
-    constexpr int T = threads_for_half<M>();
-    const size_t smem = sizeof(float2) * M + kTabSmem;
-    cudaError_t e;
-    if (p.storage == SARBP_STORE_C64) {
-        auto k = rc_inverse2_kernel<M, T, SARBP_STORE_C64>;
-        e = allow_dynamic_smem(reinterpret_cast<const void *>(k));
-        if (e != cudaSuccess || t_prepare) return e;
-        k<<<2 * p.np * p.L, T, smem, s>>>(p.ns, p.L, p.nbins, spec, etab, bound2, scale, out);
-    } else {
-        auto k = rc_inverse2_kernel<M, T, SARBP_STORE_C32H>;
-        e = allow_dynamic_smem(reinterpret_cast<const void *>(k));
-        if (e != cudaSuccess || t_prepare) return e;
-        k<<<2 * p.np * p.L, T, smem, s>>>(p.ns, p.L, p.nbins, spec, etab, bound2, scale, out);
-    }
     return cudaGetLastError();
 }
 
@@ -393,11 +365,9 @@ cudaError_t launch_rc_forward(const RcPlan &p, const float2 *echo, const float2 
                               const float2 *etab, float2 *spec, float *scale, cudaStream_t s) {
     if (p.np <= 0) return cudaSuccess;
     if (p.L < 1 || p.L > 16) return cudaErrorInvalidValue;
-    if (p.nfft >= SARBP_RC_SPLIT_MIN && p.nfft >= 8192) {
+    if (p.nfft == 32768) {
         if (!p.bound2 && !t_prepare) return cudaErrorInvalidValue;
-        if (p.nfft == 32768) return fwd2<16384>(p, echo, filt, etab, spec, p.bound2, s);
-        if (p.nfft == 16384) return fwd2<8192>(p, echo, filt, etab, spec, p.bound2, s);
-        if (p.nfft == 8192) return fwd2<4096>(p, echo, filt, etab, spec, p.bound2, s);
+        return fwd2<16384>(p, echo, filt, etab, spec, p.bound2, s);
     }
 #define SARBP_FWD(N) fwd_n<N>(p, echo, filt, etab, spec, scale, s)
     SARBP_RC_SWITCH(p.nfft, SARBP_FWD)
@@ -408,14 +378,12 @@ cudaError_t launch_rc_inverse(const RcPlan &p, const float2 *spec, const float2 
                               const float *scale, void *out, cudaStream_t s) {
     if (p.np <= 0) return cudaSuccess;
     if (p.L < 1 || p.L > 16) return cudaErrorInvalidValue;
-    if (p.nfft >= SARBP_RC_SPLIT_MIN && p.nfft >= 8192) {
+    float *sc = const_cast<float *>(scale);
+    if (p.nfft == 32768) {
         if (!p.bound2 && !t_prepare) return cudaErrorInvalidValue;
-        float *sc = const_cast<float *>(scale);
-        if (p.nfft == 32768) return inv2<16384>(p, spec, etab, p.bound2, sc, out, s);
-        if (p.nfft == 16384) return inv2<8192>(p, spec, etab, p.bound2, sc, out, s);
-        if (p.nfft == 8192) return inv2<4096>(p, spec, etab, p.bound2, sc, out, s);
+        return inv_n<32768>(p, spec, etab, p.bound2, sc, out, s);
     }
-#define SARBP_INV(N) inv_n<N>(p, spec, etab, scale, out, s)
+#define SARBP_INV(N) inv_n<N>(p, spec, etab, nullptr, sc, out, s)
     SARBP_RC_SWITCH(p.nfft, SARBP_INV)
 #undef SARBP_INV
 }

@@ -42,15 +42,9 @@ namespace {
 
 // ------------------------------------------------------------------ DFT rows
 
-#ifndef SARBP_DFT_T8192
-#define SARBP_DFT_T8192 512
-#endif
-#ifndef SARBP_DFT_T4096
-#define SARBP_DFT_T4096 512
-#endif
 template <int N>
 constexpr int dft_threads() {
-    return N >= 16384 ? 1024 : (N >= 8192 ? SARBP_DFT_T8192 : (N >= 4096 ? SARBP_DFT_T4096 : (N >= 512 ? N / 8 : 64)));
+    return N >= 16384 ? 1024 : (N >= 8192 ? 512 : (N >= 4096 ? 512 : (N >= 512 ? N / 8 : 64)));
 }
 
 // Element i of the transformed row b: the row itself, or (fused padding and
@@ -71,11 +65,11 @@ __global__ void __launch_bounds__(T, (fft_min_blocks<N, T>())) dft_pow2_kernel(f
     float2 *row = data + (size_t)blockIdx.x * ld;
     if constexpr (stage_radix<N, T, 1>() == N) {  // one stage: through shared memory
         const Etab E = load_etab<N, T>(sm, etab, 1);
-        for (int i = threadIdx.x; i < N; i += T) sm[sw(i)] = dft_input(io, row, blockIdx.x, i);
+        for (int i = threadIdx.x; i < N; i += T) sm[sw<N, T>(i)] = dft_input(io, row, blockIdx.x, i);
         __syncthreads();
         fft_smem<N, T, INV>(sm, E);
         for (int i = threadIdx.x; i < N; i += T) {
-            const float2 v = sm[sw(i)];
+            const float2 v = sm[sw<N, T>(i)];
             row[i] = make_float2(v.x * scale, v.y * scale);
         }
         return;
@@ -115,24 +109,23 @@ __global__ void __launch_bounds__(T, (fft_min_blocks<M, T>())) dft_bluestein_ker
                 if (!INV) w.y = -w.y;
                 x = cmul(dft_input(io, row, blockIdx.x, i), w);
             }
-            sm[sw(i)] = x;
+            sm[sw<M, T>(i)] = x;
         }
         __syncthreads();
         fft_smem<M, T, false>(sm, E);
-        for (int i = threadIdx.x; i < M; i += T) sm[sw(i)] = cmul(sm[sw(i)], __ldg(&kspec[i]));
+        for (int i = threadIdx.x; i < M; i += T) sm[sw<M, T>(i)] = cmul(sm[sw<M, T>(i)], __ldg(&kspec[i]));
         __syncthreads();
         fft_smem<M, T, true>(sm, E);
         for (int i = threadIdx.x; i < n; i += T) {
             float2 w = __ldg(&chirp[i]);
             if (!INV) w.y = -w.y;
-            const float2 y = cmul(sm[sw(i)], w);
+            const float2 y = cmul(sm[sw<M, T>(i)], w);
             row[i] = make_float2(y.x * scale, y.y * scale);
         }
         return;
     } else {
     using F = FirstIn<M, T>;
-    // tables first: with the chirped inputs live through the table loads the
-    // two-CTA register budget (64) spills
+    // tables first: the chirped inputs are not live through their loads
     const Etab E = load_etab<M, T>(sm, etab, 1);
     float2 v[F::PER][F::R];
     // forward transform of the chirped row: inputs straight into registers
@@ -151,15 +144,12 @@ __global__ void __launch_bounds__(T, (fft_min_blocks<M, T>())) dft_bluestein_ker
         }
     fft_io<M, T, false>(sm, E, v, SmemSink{});
     // times the kernel spectrum on the way into the inverse's first stage.
-    // At the two-CTA budget of 64 registers this keeps about 120 bytes per
-    // thread in (L1-resident) local memory; still faster than a separate
-    // multiply pass through shared memory: 1.080 vs 1.129 ms per omega-K image.
 #pragma unroll
     for (int b = 0; b < F::PER; ++b)
 #pragma unroll
         for (int r = 0; r < F::R; ++r) {
             const int i = F::point(b, r);
-            v[b][r] = F::live(b) ? cmul(sm[sw(i)], __ldg(&kspec[i])) : make_float2(0.f, 0.f);
+            v[b][r] = F::live(b) ? cmul(sm[sw<M, T>(i)], __ldg(&kspec[i])) : make_float2(0.f, 0.f);
         }
     __syncthreads();  // every point read before the first stage overwrites it
     fft_io<M, T, true>(sm, E, v, [&](int i, float2 x) {
@@ -204,14 +194,14 @@ __global__ void __launch_bounds__(T, (C <= 2 ? 2 : 1)) dft_cols_kernel(const flo
     for (int it = 0; it < N * C / T; ++it) {
         const int e = threadIdx.x + it * T;
         const int c = e % C, i = e / C, col = c0 + c;
-        sm[c * CS + sw(i)] = col < ncols ? in[(size_t)i * ncols + col] : make_float2(0.f, 0.f);
+        sm[c * CS + sw<N, T>(i)] = col < ncols ? in[(size_t)i * ncols + col] : make_float2(0.f, 0.f);
     }
     __syncthreads();  // also publishes the W tables
     StagesBatched<N, T, INV, 1, C, CS>::run(sm, E);
     for (int e = threadIdx.x; e < N * C; e += T) {
         const int c = e % C, i = e / C, col = c0 + c;
         if (col < ncols) {
-            const float2 v = sm[c * CS + sw(i)];
+            const float2 v = sm[c * CS + sw<N, T>(i)];
             out[(size_t)i * ncols + col] = make_float2(v.x * scale, v.y * scale);
         }
     }
