@@ -42,9 +42,12 @@ namespace {
 
 // ------------------------------------------------------------------ DFT rows
 
+// 8192 points: 256 threads (32-32-8, no spill at 128 registers) against 512
+// (16-16-16-2, 136 bytes of the Bluestein kernel spilled at 64): omega-K image
+// 791 -> 762 us.
 template <int N>
 constexpr int dft_threads() {
-    return N >= 16384 ? 1024 : (N >= 8192 ? 512 : (N >= 4096 ? 512 : (N >= 512 ? N / 8 : 64)));
+    return N >= 16384 ? 1024 : (N >= 8192 ? 256 : (N >= 4096 ? 512 : (N >= 512 ? N / 8 : 64)));
 }
 
 // Element i of the transformed row b: the row itself, or (fused padding and
