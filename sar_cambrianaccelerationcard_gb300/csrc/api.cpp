@@ -9,6 +9,8 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
+#include <chrono>
 #include <cmath>
 #include <complex>
 #include <cstdarg>
@@ -108,8 +110,10 @@ struct sarbp_ctx {
     DftCache dft[4];
     uint64_t dft_clock = 0;
     RcTables tables;
-    DevBuf ext;                              // planning extremes [5] (FP64 bits, nonfinite flag)
-    unsigned long long *ext_host = nullptr;  // pinned host copy of ext
+    DevBuf ext;                              // planning extremes: the reduction's state words
+    unsigned long long *ext_host = nullptr;  // its result (pinned, written by the kernel), sequence number last
+    unsigned long long ext_seq = 0;          // sequence number of the last reduction queued
+    bool ext_pending = false;                // queued and not waited for yet
     cudaEvent_t ev_ext = nullptr;
     cudaStream_t copy_stream = nullptr;      // chunked echo uploads beside range compression
     cudaEvent_t ev_copy = nullptr;
@@ -397,22 +401,40 @@ sarbp_status check_grid(sarbp_ctx *ctx, const sarbp_grid *g) {
 // Geometry extremes for planning from a device-resident APC: a reduction on the
 // stream (after the work already queued there, which may produce the APC), then
 // a wait for its 40-byte result only.  Fails on a non-finite APC coordinate.
-// Planning extremes in two halves: queue the reduction and its 40-byte
-// read-back on s, then (after any work that does not need the plan has been
-// queued behind it) wait for the read-back alone.
+// Planning extremes in two halves: queue the reduction on s, then (after any
+// work that does not need the plan has been queued behind it) wait for its
+// result alone, which the kernel writes to host memory.
 sarbp_status extremes_enqueue(sarbp_ctx *ctx, const double *apc_dev, int np, const sarbp_grid *g, cudaStream_t s) {
     Range range("sarbp: planning extremes");
-    SARBP_CUDA(ctx, sarbp::launch_bp_extremes(apc_dev, np, *g, ctx->ext.as<unsigned long long>(), s),
+    // a call that failed between the two halves may have left its reduction
+    // running (or, under stream capture, never started it)
+    if (ctx->ext_pending && cudaEventSynchronize(ctx->ev_ext) != cudaSuccess) cudaGetLastError();
+    SARBP_CUDA(ctx, sarbp::launch_bp_extremes(apc_dev, np, *g, ctx->ext.as<unsigned long long>(), ctx->ext_host,
+                                              ++ctx->ext_seq, s),
                "planning extremes");
-    ctx->launches += np > 0 ? 2 : 1;
-    SARBP_CUDA(ctx, cudaMemcpyAsync(ctx->ext_host, ctx->ext.ptr, 5 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s),
-               "read planning extremes");
+    ctx->launches += 1;
+    ctx->ext_pending = true;
     SARBP_CUDA(ctx, cudaEventRecord(ctx->ev_ext, s), "read planning extremes");
     return SARBP_OK;
 }
 
+// The result usually lands within microseconds (small calls wait for nothing
+// else): poll it for kExtPollNs, and only then sleep on the event, which takes
+// tens of microseconds to wake.  A stream still busy with an earlier
+// back-projection thus costs a core no more than the poll.
+constexpr long long kExtPollNs = 60000;
 sarbp_status extremes_wait(sarbp_ctx *ctx, sarbp::BpExtremes &e) {
-    SARBP_CUDA(ctx, cudaEventSynchronize(ctx->ev_ext), "read planning extremes");
+    const volatile unsigned long long *seq = &ctx->ext_host[5];
+    const auto until = std::chrono::steady_clock::now() + std::chrono::nanoseconds(kExtPollNs);
+    while (*seq != ctx->ext_seq) {
+        if (std::chrono::steady_clock::now() < until) continue;
+        const cudaError_t err = cudaEventSynchronize(ctx->ev_ext);
+        ctx->ext_pending = false;
+        if (err != cudaSuccess) return cuda_fail(ctx, err, "read planning extremes");
+        if (*seq != ctx->ext_seq) return fail(ctx, SARBP_ERR_INTERNAL, "planning extremes did not arrive");
+    }
+    std::atomic_thread_fence(std::memory_order_acquire);
+    ctx->ext_pending = false;
     double v[4];  // squared range extremes, cosines
     std::memcpy(v, ctx->ext_host, sizeof v);
     sarbp::ext_ranges(v[0], v[1], e);
@@ -689,7 +711,11 @@ sarbp_status sarbp_create(sarbp_ctx **out, int device) {
     ok = ok && cudaEventCreateWithFlags(&ctx->ev_copy, cudaEventDisableTiming) == cudaSuccess;
     ok = ok && cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking) == cudaSuccess;
     ok = ok && cudaMallocHost(reinterpret_cast<void **>(&ctx->ext_host), 8 * sizeof(unsigned long long)) == cudaSuccess;
-    ok = ok && ctx->ext.ensure(8 * sizeof(unsigned long long)) == cudaSuccess;
+    if (ok) std::memset(ctx->ext_host, 0, 8 * sizeof(unsigned long long));
+    unsigned long long ext_state[6];
+    sarbp::bp_extremes_state_init(ext_state);
+    ok = ok && ctx->ext.ensure(sizeof ext_state) == cudaSuccess &&
+         cudaMemcpy(ctx->ext.ptr, ext_state, sizeof ext_state, cudaMemcpyHostToDevice) == cudaSuccess;
     ok = ok && ctx->errword.ensure(sizeof(unsigned)) == cudaSuccess && ctx->power.ensure(sizeof(double)) == cudaSuccess;
     ok = ok && cudaMemset(ctx->errword.ptr, 0, sizeof(unsigned)) == cudaSuccess;
     if (!ok) {

@@ -267,11 +267,14 @@ inline void ext_ranges(double r2min, double r2max, BpExtremes &e) {
 void ext_axes(const sarbp_grid &g, double *lux, double *luy);
 // Host reduction over apc [np][3] (host memory).
 void bp_extremes_host(const double *apc, int np, const sarbp_grid &g, BpExtremes &e);
-// Device reduction over apc [np][3] (device memory) into out[0..3] (the four
-// extremes as FP64 bit patterns) and out[4] (nonfinite flag): launches the
-// initialisation and the reduction on `s`.
-cudaError_t launch_bp_extremes(const double *apc, int np, const sarbp_grid &g, unsigned long long *out,
-                               cudaStream_t s);
+// Device reduction over apc [np][3] (device memory, np > 0) on `s`: result[0..3]
+// (device-mapped host memory) receive the four extremes as FP64 bit patterns
+// (squared ranges first), result[4] the nonfinite flag and then result[5] `seq`.
+// state: six words of device memory, set once from bp_extremes_state_init; each
+// launch leaves them so, and no two launches on one state may overlap.
+void bp_extremes_state_init(unsigned long long (&state)[6]);
+cudaError_t launch_bp_extremes(const double *apc, int np, const sarbp_grid &g, unsigned long long *state,
+                               unsigned long long *result, unsigned long long seq, cudaStream_t s);
 
 // Host planning (plan.cpp): fills every BpPlan field that does not depend on
 // buffers (geometry, constants, tile height, window, series terms, segments
