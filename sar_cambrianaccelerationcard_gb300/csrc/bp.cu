@@ -1251,18 +1251,22 @@ size_t bp_smem_bytes(int storage, int win, int chunk) {
 // in FP32 (coordinates as float pairs, so differences keep FP32 relative
 // accuracy) finds the block's extremes, and only the points within the FP32
 // error of one of them are evaluated in FP64, by the host's own expressions.
-// FP32 errors: squared range 11 ulp (7e-7 relative, kExtR2 is over 5 times that),
-// cosine 1.6e-6 absolute (kExtCos 5 times).  Points whose distance is not
-// well above the rounding of the coordinates, or whose FP32 terms are not
-// ordinary numbers, are always evaluated.  Min and max do not depend on the
+// The largest cosine is the smallest sine, |axis x w| / (|axis| R), which FP32
+// separates to a microradian even where the cosines all round to 1 (a short
+// aperture at broadside: half its points lie within FP32 rounding of the largest
+// cosine, and evaluating them took 28 us at 256 pulses).  FP32 errors: squared
+// range 11 ulp (7e-7 relative, kExtR2 is over 5 times that), sine 9e-7 absolute
+// (kExtSin 4 times).  Points whose distance is not well above the rounding of
+// the coordinates, or whose FP32 terms are not ordinary numbers, are always
+// evaluated.  Min and max do not depend on the
 // order, so the bits are the host's.  The last block to finish hands the
 // result to the host (mapped memory, `seq` last) and resets the state for the
 // next call: one launch, no copy.  With the polled result (extremes_wait in
-// api.cpp) a back-projection call of 256 pulses onto 128^2 pixels takes 70 us
-// instead of 129, config 1 as one call 237 instead of 267, a projection of 2048
+// api.cpp) a back-projection call of 256 pulses onto 128^2 pixels takes 63 us
+// instead of 129, config 1 as one call 235 instead of 267, a projection of 2048
 // pulses 1.68 ms instead of 1.73.
 constexpr int kExtThreads = 64;
-constexpr float kExtR2 = 4e-6f, kExtCos = 8e-6f;
+constexpr float kExtR2 = 4e-6f, kExtSin = 4e-6f;
 struct ExtAxes {
     double len[2];     // |ux|, |uy|
     float unit[2][3];  // ux / |ux|, uy / |uy| (0 for an axis of length 0)
@@ -1305,7 +1309,12 @@ __global__ void __launch_bounds__(kExtThreads)
         ext_split(a[d], ah[d], al[d]);
         size = fmaxf(size, fabsf(ah[d]));
     }
-    auto terms = [&](int k, float &r2, float &qx, float &qy, float &always) {
+    // |unit x w| / R: the sine of the angle to an axis
+    auto sine = [](const float *e, const float *w, float inv) {
+        const float a = e[1] * w[2] - e[2] * w[1], b = e[2] * w[0] - e[0] * w[2], c = e[0] * w[1] - e[1] * w[0];
+        return sqrtf(fmaf(a, a, fmaf(b, b, c * c))) * inv;
+    };
+    auto terms = [&](int k, float &r2, float &sx, float &sy, float &always) {
         float w[3], s = size;
         for (int d = 0; d < 3; ++d) {
             w[d] = (Ph[k][d] - ah[d]) + (Pl[k][d] - al[d]);
@@ -1313,47 +1322,58 @@ __global__ void __launch_bounds__(kExtThreads)
         }
         r2 = fmaf(w[0], w[0], fmaf(w[1], w[1], w[2] * w[2]));
         const float inv = rsqrtf(r2);
-        qx = fabsf(fmaf(ax.unit[0][0], w[0], fmaf(ax.unit[0][1], w[1], ax.unit[0][2] * w[2]))) * inv;
-        qy = fabsf(fmaf(ax.unit[1][0], w[0], fmaf(ax.unit[1][1], w[1], ax.unit[1][2] * w[2]))) * inv;
+        sx = sine(ax.unit[0], w, inv);
+        sy = sine(ax.unit[1], w, inv);
         always = fmaxf(1e-30f, s * 2.4e-7f * (s * 2.4e-7f));
     };
-    float m[4] = {3.4e38f, 0.f, 0.f, 0.f};  // min r2, max r2, max cosines (fminf / fmaxf drop NaN)
+    float m[4] = {0.f, 3.4e38f, 3.4e38f, 3.4e38f};  // max r2, min r2, min sines (fminf / fmaxf drop NaN)
     if (live) {
 #pragma unroll 3
         for (int v = 0; v < kLattice; ++v) {
-            float r2, qx, qy, always;
-            terms(u * kLattice + v, r2, qx, qy, always);
-            m[0] = fminf(m[0], r2);
-            m[1] = fmaxf(m[1], r2);
-            m[2] = fmaxf(m[2], qx);
-            m[3] = fmaxf(m[3], qy);
+            float r2, sx, sy, always;
+            terms(u * kLattice + v, r2, sx, sy, always);
+            m[0] = fmaxf(m[0], r2);
+            m[1] = fminf(m[1], r2);
+            m[2] = fminf(m[2], sx);
+            m[3] = fminf(m[3], sy);
         }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-        m[0] = fminf(m[0], __shfl_xor_sync(0xffffffffu, m[0], o));
+        m[0] = fmaxf(m[0], __shfl_xor_sync(0xffffffffu, m[0], o));
 #pragma unroll
-        for (int k = 1; k < 4; ++k) m[k] = fmaxf(m[k], __shfl_xor_sync(0xffffffffu, m[k], o));
+        for (int k = 1; k < 4; ++k) m[k] = fminf(m[k], __shfl_xor_sync(0xffffffffu, m[k], o));
     }
     if ((t & 31) == 0)
         for (int k = 0; k < 4; ++k) red[k][t >> 5] = m[k];
     __syncthreads();
     for (int w = 0; w < kExtThreads / 32; ++w) {
-        m[0] = fminf(m[0], red[0][w]);
-        for (int k = 1; k < 4; ++k) m[k] = fmaxf(m[k], red[k][w]);
+        m[0] = fmaxf(m[0], red[0][w]);
+        for (int k = 1; k < 4; ++k) m[k] = fminf(m[k], red[k][w]);
     }
     if (live) {
-        const float lo = m[0] * (1.f + kExtR2), hi = m[1] * (1.f - kExtR2), cx = m[2] - kExtCos, cy = m[3] - kExtCos;
+        const float hi = m[0] * (1.f - kExtR2), lo = m[1] * (1.f + kExtR2), ex = m[2] + kExtSin, ey = m[3] + kExtSin;
         ExtAcc acc;
         ext_acc_init(acc);
         bool any = false;
 #pragma unroll 1
         for (int v = 0; v < kLattice; ++v) {
-            float r2, qx, qy, always;
-            terms(u * kLattice + v, r2, qx, qy, always);
-            // false only for ordinary numbers clear of every extreme
-            if (!(r2 > lo) || !(r2 < hi) || !(qx < cx) || !(qy < cy) || !(r2 > always)) {
-                ext_acc_point(acc, g, ax.len[0], ax.len[1], P[u * kLattice + v], a);
+            float r2, sx, sy, always;
+            terms(u * kLattice + v, r2, sx, sy, always);
+            // false only for ordinary numbers clear of the extreme; a cosine's
+            // quotient and square root only where it may be the largest
+            const bool all = !(r2 > always);
+            const bool range = all || !(r2 > lo) || !(r2 < hi);
+            const bool cos_x = all || !(sx > ex), cos_y = all || !(sy > ey);
+            if (range || cos_x || cos_y) {
+                double r2d, nx, ny;
+                ext_terms(g, P[u * kLattice + v], a, r2d, nx, ny);
+                acc.r2min = fmin(acc.r2min, r2d);
+                acc.r2max = fmax(acc.r2max, r2d);
+                if (r2d > 0) {
+                    if (cos_x && ax.len[0] > 0) ext_cos(acc.cx, nx, r2d, ax.len[0]);
+                    if (cos_y && ax.len[1] > 0) ext_cos(acc.sy, ny, r2d, ax.len[1]);
+                }
                 any = true;
             }
         }
