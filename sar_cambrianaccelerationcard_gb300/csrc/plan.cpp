@@ -252,6 +252,7 @@ bool plan_bp(int sms, const sarbp_radar &r, const sarbp_rc_view &rc, const BpExt
     const int tiles = ((g.nx + tx - 1) / tx) * ((g.ny + ty - 1) / ty);
     const int npl = pulses_per_launch > 0 ? pulses_per_launch : np;
     p.segments = bp_choose_segments(tiles, npl, (long long)g.nx * g.ny, sms, tune ? tune->bp_segments : 0);
+    if (!(tune && tune->bp_segments)) p.segments = bp_fill_segments(tiles, npl, sms, p.segments);
     return true;
 }
 
@@ -282,6 +283,22 @@ int bp_choose_segments(int tiles, int npl, long long npix, int sms, int force) {
         if ((long long)tiles * s >= target) break;
     }
     return best;
+}
+
+// Small images: where the rule above splits the pulses but its segments leave SMs
+// without a CTA, more of them, down to one chunk of pulses each, until every SM
+// has one (256 pulses onto 128^2 pixels: 8 tiles x 4 segments 22 us, x 16
+// 10.8 us).  Their partial images are small: fewer tiles than SMs.  Apertures
+// the rule keeps in one segment (under 128 pulses) stay there: their sums are
+// one launch in pulse order, without a reduction.
+int bp_fill_segments(int tiles, int npl, int sms, int segments) {
+    const int kc = bp_max_chunk();
+    if (segments < 2) return segments;
+    for (int s = segments + 1; s <= 64 && (long long)tiles * segments < sms && npl / s >= kc; ++s) {
+        const int pps = ((npl + s - 1) / s + kc - 1) / kc * kc;  // as the launch rounds it
+        if ((long long)(s - 1) * pps < npl) segments = s;        // no empty segment
+    }
+    return segments;
 }
 
 void rc_tables_fill(const sarbp_radar &r, const sarbp_rc_layout &lay, std::complex<double> *h, float2 *filt,

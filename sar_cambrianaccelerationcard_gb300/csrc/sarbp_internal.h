@@ -306,6 +306,8 @@ int bp_max_chunk();  // largest pulse chunk (16); the planner may choose 8 or 4
 // (at least 12 waves of CTAs where the pulses allow; at least 4 chunks per
 // segment; partial images within 1 GiB); `force` in 1..64 overrides.
 int bp_choose_segments(int tiles, int npl, long long npix, int sms, int force = 0);
+// more segments for calls that would leave SMs without a CTA (plan.cpp)
+int bp_fill_segments(int tiles, int npl, int sms, int segments);
 
 // ---------------------------------------------------------------- echo synthesis
 cudaError_t launch_echo_synth(const double *apc, int np, int ns, const sarbp_target *tg, int nt,
