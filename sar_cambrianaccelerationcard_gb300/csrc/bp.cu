@@ -105,27 +105,21 @@ constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23: adding it rounds to an int
 constexpr unsigned kMagicBitsShift4 = 0x4B400000u << 4;
 
 struct __align__(16) Prm {
-    // back-projection, split arithmetic: each constant once (the packed
-    // operations read a scalar as both halves); projection: each constant twice,
-    // so a 16-byte load yields two packed operands
-    float4 k0;     // c1, c2, c3, c4      projection: c1, c1, c2, c2     FP32: apc x, y, z, bin offset
-    float4 k1;     // bin', phT, A, B     projection: c3, c3, c4, c4
-    float4 k2;     // LIN: PX, PY, 0, 0   projection: bin', bin', phT, phT
-    float4 k3;     // -                   projection: A, A, B, B
+    // split arithmetic: each constant once, the packed operations read a scalar
+    // as both halves
+    float4 k0;     // c1, c2, c3, c4 (LIN: c1, d2, d3, d4)      FP32: apc x, y, z, bin offset
+    float4 k1;     // bin', phT, A, B (LIN: A c1, B c1)          FP32: phase correction
+    float2 k2;     // LIN: the phase increments per pixel step PX, PY
     double ax, ay, az;  // FP64: APC position
     double dr, dph;     // FP64: per-pulse range (m) and phase (rad) corrections
     int ws;        // first bin of the window
     int lo, hi;    // copied part of the window [lo, hi) relative to ws
     float scale;   // FP16 storage scale
     int need;      // (M, d) pairs [0, need) any pixel of the tile reads (the rest are not converted)
+    int unused[4];
 };
-
-// Linear-term projection: the phase increments per pixel step,
-// (PX, PX, PY, PY), in the 16 bytes of the FP64-only ax, ay (offset 64,
-// 16-byte aligned), so the record keeps its size.
-__device__ __forceinline__ float4 &prm_k4(Prm &q) { return *reinterpret_cast<float4 *>(&q.ax); }
-__device__ __forceinline__ const float4 &prm_k4(const Prm &q) { return *reinterpret_cast<const float4 *>(&q.ax); }
-static_assert(offsetof(Prm, ax) % 16 == 0 && offsetof(Prm, az) - offsetof(Prm, ax) == 16, "k4 slot");
+// the planner's shared-memory bounds (which windows it accepts) count 128 bytes
+static_assert(sizeof(Prm) == 128, "Prm size");
 
 __device__ __forceinline__ float4 lds128(unsigned addr) {
     float4 v;
@@ -183,7 +177,6 @@ __device__ __forceinline__ void sts2x2(void *p, f2 a, f2 b) {
 __device__ __forceinline__ void lds2x2_at(unsigned addr, f2 &a, f2 &b) {
     asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "r"(addr));
 }
-__device__ __forceinline__ void lds2x2(const void *p, f2 &a, f2 &b) { lds2x2_at(smem_addr(p), a, b); }
 
 struct Smem {
     float4 *staged;      // [2][chunk][win]
@@ -262,7 +255,7 @@ __device__ __noinline__ void drain_after_timeout(const BpPlan &P, uint64_t *bars
 // by one warp (a lane per pulse), which arrives once on the stage's barrier.
 // `fault` (tests only) arms the arrival with kFaultBytes that no copy delivers,
 // so the phase cannot complete and the staging warps' bounded wait runs out.
-template <int MODE, int STORE, int PIX, bool LIN, bool ADJ>
+template <int MODE, int STORE, int PIX, bool LIN>
 __device__ __forceinline__ void produce(const BpPlan &P, const Smem &S, int stage, int p0, int count,
                                         const TileGeo &T, bool fault) {
     constexpr int kTileY = 8 * PIX;
@@ -332,29 +325,16 @@ __device__ __forceinline__ void produce(const BpPlan &P, const Smem &S, int stag
                     const ff kh = {0.5f * P.kp_h, 0.5f * P.kp_l};  // 2 pi fc / c
                     const float pxr = ff_mod_2pi(ff_mul(ff_mul(kh, uxw), invR));
                     const float pyr = ff_mod_2pi(ff_mul(ff_mul(kh, uyw), invR));
-                    if constexpr (ADJ) {
-                        q.k0 = make_float4(c1, c1, d2, d2);
-                        q.k1 = make_float4(d3, d3, d4, d4);
-                        q.k2 = make_float4(bb, bb, phT, phT);
-                        q.k3 = make_float4(A * c1, A * c1, B * c1, B * c1);
-                        prm_k4(q) = make_float4(pxr, pxr, pyr, pyr);
-                    } else {
-                        q.k0 = make_float4(c1, d2, d3, d4);
-                        q.k1 = make_float4(bb, phT, A * c1, B * c1);
-                        q.k2 = make_float4(pxr, pyr, 0.f, 0.f);
-                    }
-                } else if constexpr (!ADJ) {
+                    q.k0 = make_float4(c1, d2, d3, d4);
+                    q.k1 = make_float4(bb, phT, A * c1, B * c1);
+                    q.k2 = make_float2(pxr, pyr);
+                } else {
                     q.k0 = make_float4(c1, c2, c3, c4);
                     q.k1 = make_float4(bb, phT, A, B);
-                } else {
-                    q.k0 = make_float4(c1, c1, c2, c2);
-                    q.k1 = make_float4(c3, c3, c4, c4);
-                    q.k2 = make_float4(bb, bb, phT, phT);
-                    q.k3 = make_float4(A, A, B, B);
                 }
             } else {  // inert pulse: every pixel reads the centre bin of an all-zero window
-                q.k0 = q.k1 = q.k2 = q.k3 = make_float4(0.f, 0.f, 0.f, 0.f);
-                if constexpr (LIN) prm_k4(q) = make_float4(0.f, 0.f, 0.f, 0.f);
+                q.k0 = q.k1 = make_float4(0.f, 0.f, 0.f, 0.f);
+                q.k2 = make_float2(0.f, 0.f);
             }
         } else {
             const double ax = __ldg(&P.apc[3 * p]), ay = __ldg(&P.apc[3 * p + 1]), az = __ldg(&P.apc[3 * p + 2]);
@@ -516,14 +496,15 @@ __device__ __forceinline__ void flush_projection(const BpPlan &P, const Smem &S,
 // LIN: the linear-term phase (as the back-projection's LIN loop), the weight's
 // phase added to it the same way.
 template <int NTERMS, int PIX, bool LIN>
-__device__ __forceinline__ void project_chunk(const Smem &S, int stage, int count, int win, unsigned sbase, int cen,
-                                              f2 XC2, const f2 (&YC2)[PIX / 2], const f2 (&QQ2)[PIX / 2], f2 BPM2,
+__device__ __forceinline__ void project_chunk(const Smem &S, int stage, int count, int win, unsigned stg, int cen,
+                                              float xc, const f2 (&YC2)[PIX / 2], const f2 (&QQ2)[PIX / 2], f2 BPM2,
                                               f2 KH2, f2 KL2, const f2 (&TH2)[PIX / 2], const float (&wm)[PIX],
-                                              f2 X2C2, const f2 (&Y2C2)[LIN ? PIX / 2 : 1], float *red) {
+                                              const f2 (&Y2C2)[LIN ? PIX / 2 : 1], float *red) {
     const int lane = threadIdx.x & 31;
     const bool hi16 = (lane & 16) != 0, hi8 = (lane & 8) != 0;
-    f2 MP = pk2(kMagic + (float)cen, kMagic + (float)cen);
-    const f2 WIN2 = pk2((float)win, (float)win);
+    const f2 XC2 = bc2(xc);
+    float mp = kMagic + (float)(int)((stg >> 4) + cen);  // the window middle's 16-byte slot
+    const float winf = (float)win;
 #pragma unroll 1
     for (int pl = 0; pl < count; pl += 2) {
         float tr[2] = {0.f, 0.f}, ti[2] = {0.f, 0.f};
@@ -531,31 +512,27 @@ __device__ __forceinline__ void project_chunk(const Smem &S, int stage, int coun
         for (int u2 = 0; u2 < 2; ++u2) {
             if (u2 == 1 && pl + 1 >= count) break;  // odd tail: pulse-uniform
             const Prm &q = S.prm[stage * kChunk + pl + u2];
-            // k0..k3 (and k4 for LIN) as the producer wrote them: (C1, C2 | D2),
-            // (C3 | D3, C4 | D4), (BT, PHT), (A | A c1, B | B c1), (PX, PY)
-            f2 C1, C2, C3, C4, BT, PHT, AA, BB, PX, PY;
-            lds2x2(&q.k0, C1, C2);
-            lds2x2(&q.k1, C3, C4);
-            lds2x2(&q.k2, BT, PHT);
-            lds2x2(&q.k3, AA, BB);
-            f2 PHX = PHT;
+            const float4 v0 = lds128(smem_addr(&q.k0)), v1 = lds128(smem_addr(&q.k1));
+            const f2 C1 = bc2(v0.x), C2 = bc2(v0.y), C3 = bc2(v0.z), C4 = bc2(v0.w);  // LIN: C1, D2, D3, D4
+            const f2 BT = bc2(v1.x), PHT = bc2(v1.y), AA = bc2(v1.z), BB = bc2(v1.w);
+            f2 PHX = PHT, PY = PHT;
             if constexpr (LIN) {
-                lds2x2(&prm_k4(q), PX, PY);
-                PHX = ffma2(X2C2, PX, PHT);
+                const float2 v2 = q.k2;
+                PHX = bc2(fmaf(2.f * xc, v2.x, v1.y));
+                PY = bc2(v2.y);
             }
-            const f2 XA = fmul2(XC2, AA);
 #pragma unroll
             for (int h = 0; h < PIX / 2; ++h) {
                 f2 b2, ph2;
                 if constexpr (LIN) {
                     const f2 qc = fmul2(QQ2[h], C1);
-                    const f2 m = ffma2(YC2[h], BB, fadd2(XA, qc));
+                    const f2 m = ffma2(YC2[h], BB, ffma2(XC2, AA, qc));
                     const f2 m2 = fmul2(m, m);
                     const f2 poly = NTERMS == 4 ? ffma2(m, ffma2(m, C4, C3), C2) : ffma2(m, C3, C2);
                     b2 = ffma2(ffma2(m2, poly, m), BPM2, BT);
                     ph2 = fadd2(ffma2(ffma2(m2, poly, qc), KH2, ffma2(Y2C2[h], PY, PHX)), TH2[h]);
                 } else {
-                    const f2 n = ffma2(YC2[h], BB, fadd2(XA, QQ2[h]));
+                    const f2 n = ffma2(YC2[h], BB, ffma2(XC2, AA, QQ2[h]));
                     f2 poly = NTERMS == 4 ? ffma2(n, ffma2(n, C4, C3), C2) : ffma2(n, C3, C2);
                     poly = ffma2(n, poly, C1);
                     const f2 dR = fmul2(n, poly);
@@ -569,21 +546,21 @@ __device__ __forceinline__ void project_chunk(const Smem &S, int stage, int coun
                 float bb[2], ph[2], tt[2];
                 upk2(b2, bb[0], bb[1]);
                 upk2(ph2, ph[0], ph[1]);
-                upk2(fadd2(b2, MP), tt[0], tt[1]);
+                upk2(fadd2(b2, bc2(mp)), tt[0], tt[1]);
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
                     const int j = 2 * h + u;
-                    const float4 v = lds128((__float_as_uint(tt[u]) << 4) + sbase);
-                    const float sr = fmaf(bb[u], v.z, v.x);
-                    const float si = fmaf(bb[u], v.w, v.y);
-                    float sn, cs;
+                    f2 M, D;
+                    lds2x2_at((__float_as_uint(tt[u]) << 4) - kMagicBitsShift4, M, D);
+                    float sr, si, sn, cs;
+                    upk2(ffma2(bc2(bb[u]), D, M), sr, si);
                     __sincosf(ph[u], &sn, &cs);
                     const float zr = wm[j] * cs, zi = wm[j] * sn;
                     tr[u2] = fmaf(sr, zr, fmaf(-si, zi, tr[u2]));
                     ti[u2] = fmaf(sr, zi, fmaf(si, zr, ti[u2]));
                 }
             }
-            MP = fadd2(MP, WIN2);
+            mp += winf;
         }
         float k0 = hi16 ? tr[1] : tr[0], k1 = hi16 ? ti[1] : ti[0];
         k0 += __shfl_xor_sync(0xffffffffu, hi16 ? tr[0] : tr[1], 16);
@@ -725,7 +702,6 @@ __global__ void __launch_bounds__(kThreads + 32 * helper_warps<MODE, CHECKED, PI
         if constexpr (ADJ) TH2[h] = pk2(wth[2 * h], wth[2 * h + 1]);
         if constexpr (LIN) Y2C2[h] = pk2(2.f * yc[2 * h], 2.f * yc[2 * h + 1]);
     }
-    const f2 X2C2 = pk2(2.f * xc, 2.f * xc);
 
     // Staging of chunk k: one staging warp computes the parameters and issues the
     // copies of chunk k + 1, then all of them wait for chunk k's copies and
@@ -734,7 +710,7 @@ __global__ void __launch_bounds__(kThreads + 32 * helper_warps<MODE, CHECKED, PI
     auto produce_chunk = [&](int k) {
         const int p0 = p_begin + k * chunk;
         if (k < nchunks && warp == kStager0 + (kHelpers ? 0 : k % kWarps))
-            produce<MODE, STORE, PIX, LIN, ADJ>(P, S, k % kStages, p0, min(chunk, p_end - p0), T,
+            produce<MODE, STORE, PIX, LIN>(P, S, k % kStages, p0, min(chunk, p_end - p0), T,
                                                 TESTF && P.fault_chunk == k);
     };
     auto stage_chunk = [&](int k) {
@@ -780,10 +756,9 @@ __global__ void __launch_bounds__(kThreads + 32 * helper_warps<MODE, CHECKED, PI
             if (c + 1 < nchunks) failed = !stage_chunk(c + 1);
         } else {
         const float4 *stg = S.staged + (size_t)sbuf * chunk * win;
-        const unsigned sbase = smem_addr(stg) - kMagicBitsShift4;
         if constexpr (ADJ) {
-            project_chunk<NTERMS, kPix, LIN>(S, stage, count, win, sbase, cen, XC2, YC2, QQ2, BPM2, KH2, KL2, TH2, wm,
-                                             X2C2, Y2C2, reinterpret_cast<float *>(S.red + ((c & 1) * kWarps + warp) * kChunk));
+            project_chunk<NTERMS, kPix, LIN>(S, stage, count, win, smem_addr(stg), cen, xc, YC2, QQ2, BPM2, KH2, KL2, TH2, wm,
+                                             Y2C2, reinterpret_cast<float *>(S.red + ((c & 1) * kWarps + warp) * kChunk));
         } else if (LIN && (MODE == SARBP_MODE_SPLIT || MODE == SARBP_MODE_FP16STORE)) {
             // linear-term form (large tiles): m = n / (2 R_T) centred offset, bin from
             // dR = m + m^2 poly(m), phase from the increments per pixel step (reduced
@@ -796,7 +771,7 @@ __global__ void __launch_bounds__(kThreads + 32 * helper_warps<MODE, CHECKED, PI
             for (int pl = 0; pl < count; ++pl) {
                 const Prm &q = S.prm[stage * kChunk + pl];
                 const float4 v0 = lds128(smem_addr(&q.k0)), v1 = lds128(smem_addr(&q.k1));
-                const float2 v2 = *reinterpret_cast<const float2 *>(&q.k2);
+                const float2 v2 = q.k2;
                 const f2 C1 = bc2(v0.x), D2 = bc2(v0.y), D3 = bc2(v0.z), D4 = bc2(v0.w);
                 const f2 BT = bc2(v1.x), BP = bc2(v1.w), PY = bc2(v2.y);
                 const f2 AP = bc2(v1.z);
@@ -913,7 +888,7 @@ __global__ void __launch_bounds__(kThreads + 32 * helper_warps<MODE, CHECKED, PI
                     float b = fmaf(R, bpm, k0.w);
                     b = fminf(fmaxf(b, -cenf), wmax - cenf);
                     const float t = b + mp;
-                    const float4 v = lds128((__float_as_uint(t) << 4) + sbase);
+                    const float4 v = lds128((__float_as_uint(t) << 4) + smem_addr(stg) - kMagicBitsShift4);
                     const float sr = fmaf(b, v.z, v.x);
                     const float si = fmaf(b, v.w, v.y);
                     float sn, cs;
