@@ -19,21 +19,26 @@
 //    mid_i = (s_i + s_{i+1})/2, diff_i = s_{i+1} - s_i, so one 16-byte shared load
 //    and two FMAs interpolate.  Converted windows are double-buffered: one
 //    block barrier per chunk.
-//  * Who stages (helper_warps): with 16-pulse chunks of 32 x 64 tiles, two extra
-//    warps per CTA, beside the pixel warps' loop over the chunk before.  The
-//    parameters (a float-float chain of some 400 instructions) then run once per
-//    chunk instead of in every warp, and neither they nor the conversion hold
-//    the pixel warps at the barrier.  20 warps per SM leave 96 registers, which
-//    the pixel loop needs: config 2 45.8 -> 42.6 ms, FP16 rows 3.63 -> 3.42 ms
-//    (the warps taking turns at the parameters, everyone converting: 44.8 and
-//    3.49 ms), weighted projection 1.78 -> 1.71 ms.  Where a chunk has less pixel
-//    work per staged bin (8 and 4 pulses, shorter tiles: wide windows) two warps
-//    cannot keep up, and the linear-term back-projection needs more than 96
-//    registers; there, and in the checked and comparator kernels, the pixel
-//    warps stage, each chunk's parameters by the next warp in turn.  1024 pulses
-//    onto 1024^2, helpers / none: 1.0 m pixels 1.40 / 1.35 ms, 1.4 m rotated by
-//    45 degrees 3.84 / 3.11 (3.81 before), 2.2 m onto 512^2 2.08 / 1.54 (1.85
-//    before), linear-term 0.5 m FP16 rows 1.03 / 1.00 (1.19 before).
+//  * Who stages (helper_warps).  The parameters are a float-float chain of some 400
+//    instructions; run by every warp for two pulses each, and with every warp
+//    converting, staging cost a quarter of the instructions and held the pixel
+//    warps at the barrier.
+//    - 16-pulse chunks of 32 x 64 tiles: two extra warps stage the next chunk
+//      beside the pixel warps' loop.  20 warps per SM leave 96 registers, which
+//      that loop needs.  Config 2 45.8 -> 42.5 ms, FP16 rows 3.63 -> 3.37 ms (the
+//      pixel warps staging, the parameters in turn: 44.8 and 3.49 ms), weighted
+//      projection 1.78 -> 1.71 ms.
+//    - 8- and 4-pulse chunks (wide windows, short tiles) have less pixel work per
+//      staged bin, and two warps cannot keep up with the conversion: one extra
+//      warp computes the parameters, the pixel warps convert.  1024 pulses onto
+//      1024^2 at 1.0 m, none / one / two helpers: 1.32 / 1.27 / 1.40 ms; 1.4 m
+//      rotated by 45 degrees 3.06 / 2.65 / 3.84 (3.80 with every warp preparing
+//      parameters); its projection 3.66 / 3.17; 2.2 m onto 512^2 1.50 / 1.27 /
+//      2.08 (1.84); 1200 x 1000 at 0.75 m, rotated 1.61 / 1.56.
+//    - The linear-term back-projection with 16-pulse chunks needs more than 96
+//      registers (0.37 m: 0.91 ms without a helper, 0.96 with one), and so do the
+//      FP64 and FP32 comparators; the checked kernels follow.  There the pixel
+//      warps stage, each chunk's parameters by the next warp in turn.
 //  * SPLIT arithmetic per pixel and pulse: with q the pixel offset from the tile
 //    centre, n = 2 q.w + |q|^2 (w = tile centre - APC) and the differential
 //    range dR = sqrt(R_T^2 + n) - R_T = n (c1 + n (c2 + n (c3 + n c4))) (series
@@ -92,12 +97,14 @@ constexpr int kTileX = 32;  // pixels along x (columns); tile height is 8 * PIX 
 #define SARBP_BP_PHASE_COMPENSATED 0
 #endif
 constexpr int kChunk = SARBP_BP_CHUNK;  // pulses per staged chunk (a multiple of 8)
-// Staging warps of a CTA beside its kWarps pixel warps; 0: the pixel warps stage.
+// Warps of a CTA beside its kWarps pixel warps: 2 stage whole chunks; 1 computes the
+// parameters and issues the copies, the pixel warps convert; 0: the pixel warps
+// do both, the parameters in turn.
 template <int MODE, bool CHECKED, int PIX, bool ADJ, int CHUNK, bool LIN>
 __host__ __device__ constexpr int helper_warps() {
-    return !CHECKED && (MODE == SARBP_MODE_SPLIT || MODE == SARBP_MODE_FP16STORE) && PIX == 8 && CHUNK && (ADJ || !LIN)
-               ? 2
-               : 0;
+    if (CHECKED || (MODE != SARBP_MODE_SPLIT && MODE != SARBP_MODE_FP16STORE)) return 0;
+    if (CHUNK) return PIX == 8 && (ADJ || !LIN) ? 2 : 0;
+    return 1;
 }
 static_assert(kChunk <= 32, "one staging lane per pulse of a chunk");
 constexpr int kStages = 3;  // raw-window ring depth
@@ -597,7 +604,8 @@ __global__ void __launch_bounds__(kThreads + 32 * helper_warps<MODE, CHECKED, PI
     // the linear-term form at 0.75 m, 1.38 / 1.38 / 1.35 / 1.40 at 1 m
     constexpr int kPulseUnroll = CHUNK && !LIN ? CHUNK : 4;
     constexpr int kHelpers = helper_warps<MODE, CHECKED, PIX, ADJ, CHUNK, LIN>();
-    constexpr int kStager0 = kHelpers ? kWarps : 0, kStagers = kHelpers ? kHelpers : kWarps;
+    constexpr bool kAhead = kHelpers == 2;  // the helpers stage chunk c + 1 while the pixel warps run chunk c
+    constexpr int kStager0 = kAhead ? kWarps : 0, kStagers = kAhead ? kHelpers : kWarps;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int win = P.win;
     const int chunk = CHUNK ? CHUNK : P.chunk;  // pulses per staged chunk: 16, 8 or 4 (two CTAs per SM)
@@ -703,13 +711,13 @@ __global__ void __launch_bounds__(kThreads + 32 * helper_warps<MODE, CHECKED, PI
         if constexpr (LIN) Y2C2[h] = pk2(2.f * yc[2 * h], 2.f * yc[2 * h + 1]);
     }
 
-    // Staging of chunk k: one staging warp computes the parameters and issues the
-    // copies of chunk k + 1, then all of them wait for chunk k's copies and
-    // convert them.  False when the wait ran out.
+    // Staging of chunk k: one warp computes the parameters and issues the copies of
+    // chunk k + 1, then the staging warps wait for chunk k's copies and convert
+    // them.  False when the wait ran out.
     const bool helper = kHelpers && warp >= kWarps;
     auto produce_chunk = [&](int k) {
         const int p0 = p_begin + k * chunk;
-        if (k < nchunks && warp == kStager0 + (kHelpers ? 0 : k % kWarps))
+        if (k < nchunks && warp == (kHelpers ? kWarps : k % kWarps))
             produce<MODE, STORE, PIX, LIN>(P, S, k % kStages, p0, min(chunk, p_end - p0), T,
                                                 TESTF && P.fault_chunk == k);
     };
@@ -729,12 +737,12 @@ __global__ void __launch_bounds__(kThreads + 32 * helper_warps<MODE, CHECKED, PI
     bool clamped = false;
     if (warp >= kStager0) {
         produce_chunk(0);
-        if (kHelpers && nchunks > 0) failed = !stage_chunk(0);
+        if (kAhead && nchunks > 0) failed = !stage_chunk(0);
     }
-    if (kHelpers) failed = __syncthreads_or(failed);
-    // One block barrier per chunk.  Helpers stage chunk c + 1 beside the pixel
-    // warps' chunk c and the barrier ends both; without helpers it follows chunk
-    // c's own staging.  Either way, when chunk k's copies and parameters are
+    if (kAhead) failed = __syncthreads_or(failed);
+    // One block barrier per chunk.  Two helpers stage chunk c + 1 beside the pixel
+    // warps' chunk c and the barrier ends both; otherwise it follows chunk c's own
+    // staging.  Either way, when chunk k's copies and parameters are
     // issued every warp is done with chunk k - 3 (the ring stage), and when its
     // pairs are written with chunk k - 2 (the buffer).  A wait that ran out ends
     // the loop for every warp.
@@ -745,15 +753,19 @@ __global__ void __launch_bounds__(kThreads + 32 * helper_warps<MODE, CHECKED, PI
         const int sbuf = c & 1;
         const int pc0 = p_begin + c * chunk;
         const int count = min(chunk, p_end - pc0);
-        if constexpr (!kHelpers) {
-            failed = __syncthreads_or(!stage_chunk(c));
+        if constexpr (!kAhead) {
+            bool staged = true;
+            if (kHelpers == 1 && helper) produce_chunk(c + 1);
+            else staged = stage_chunk(c);
+            failed = __syncthreads_or(!staged);
             if (failed) break;
+            if (kHelpers == 1 && helper) continue;
         }
         if constexpr (ADJ) {  // every pixel warp has finished chunk c - 1: combine its pulse sums
             if (c > 0 && warp == kStager0) flush_projection(P, S, (c - 1) & 1, pc0 - chunk, chunk, lane);
         }
         if (helper) {
-            if (c + 1 < nchunks) failed = !stage_chunk(c + 1);
+            if (kAhead && c + 1 < nchunks) failed = !stage_chunk(c + 1);
         } else {
         const float4 *stg = S.staged + (size_t)sbuf * chunk * win;
         if constexpr (ADJ) {
@@ -929,7 +941,7 @@ __global__ void __launch_bounds__(kThreads + 32 * helper_warps<MODE, CHECKED, PI
             }
         }
         }
-        if constexpr (kHelpers) failed = __syncthreads_or(failed);
+        if constexpr (kAhead) failed = __syncthreads_or(failed);
     }
 
     if (CHECKED && clamped) atomicOr(P.err, kErrIndexClamp);
@@ -941,7 +953,7 @@ __global__ void __launch_bounds__(kThreads + 32 * helper_warps<MODE, CHECKED, PI
 
     if constexpr (ADJ) {
         if (nchunks > 0) {
-            if (!kHelpers) __syncthreads();
+            if (!kAhead) __syncthreads();
             const int last = nchunks - 1;
             if (warp == kStager0)
                 flush_projection(P, S, last & 1, p_begin + last * chunk, min(chunk, p_end - p_begin - last * chunk), lane);
