@@ -117,6 +117,8 @@ struct sarbp_ctx {
     cudaEvent_t ev_ext = nullptr;
     cudaStream_t copy_stream = nullptr;      // chunked echo uploads beside range compression
     cudaEvent_t ev_copy = nullptr;
+    cudaEvent_t ev_scratch = nullptr;        // end of the last launches that use the back-projection scratch
+    cudaStream_t scratch_stream = nullptr;   // the stream they went to (compared only)
     // Buffers sized by the calls (released by sarbp_trim and sarbp_destroy).
     std::vector<DevBuf *> scratch() {
         std::vector<DevBuf *> v = {&echo,   &spec,  &rc,      &scale,   &apc,     &image,   &partial,
@@ -456,6 +458,20 @@ sarbp_status extremes_device(sarbp_ctx *ctx, const double *apc_dev, int np, cons
     return st != SARBP_OK ? st : extremes_wait(ctx, e);
 }
 
+// The pulse references, partial images and projection sums live in the context:
+// a call on another stream than the last one's waits for its launches before
+// it overwrites them.
+sarbp_status scratch_begin(sarbp_ctx *ctx, cudaStream_t s) {
+    if (ctx->scratch_stream && ctx->scratch_stream != s)
+        SARBP_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_scratch, 0), "order scratch");
+    return SARBP_OK;
+}
+sarbp_status scratch_end(sarbp_ctx *ctx, cudaStream_t s) {
+    SARBP_CUDA(ctx, cudaEventRecord(ctx->ev_scratch, s), "order scratch");
+    ctx->scratch_stream = s;
+    return SARBP_OK;
+}
+
 // Back-projection of device-resident rc + apc into a device image.
 sarbp_status bp_device(sarbp_ctx *ctx, const sarbp_radar *r, const sarbp_rc_view &rc, const double *apc_dev,
                        const sarbp::BpExtremes &ex, const sarbp_grid *g, int mode, float2 *image, int accumulate,
@@ -491,12 +507,14 @@ sarbp_status bp_device(sarbp_ctx *ctx, const sarbp_radar *r, const sarbp_rc_view
         p.partial = ctx->partial.as<float2>();
     }
     int launches = 0;
+    sarbp_status st = scratch_begin(ctx, s);
+    if (st != SARBP_OK) return st;
     cudaEventRecord(ctx->ev[2], s);
     SARBP_CUDA(ctx, sarbp::launch_bp(p, s, &launches), "back-projection launch");
     cudaEventRecord(ctx->ev[3], s);
     ctx->timed_bp = true;
     ctx->launches += launches;
-    return SARBP_OK;
+    return scratch_end(ctx, s);
 }
 
 // Weighted projection of device-resident rc + apc against a device weight
@@ -527,9 +545,11 @@ sarbp_status project_device(sarbp_ctx *ctx, const sarbp_radar *r, const sarbp_rc
     SARBP_CUDA(ctx, ctx->proj.ensure(sizeof(float2) * sarbp::bp_tiles(p) * (size_t)np), "alloc projection scratch");
     p.proj = ctx->proj.as<float2>();
     int launches = 0;
+    sarbp_status st = scratch_begin(ctx, s);
+    if (st != SARBP_OK) return st;
     SARBP_CUDA(ctx, sarbp::launch_project(p, out, s, &launches), "projection launch");
     ctx->launches += launches;
-    return SARBP_OK;
+    return scratch_end(ctx, s);
 }
 
 // Device-side inputs of a back-projection-type call (uploads of host arrays
@@ -714,6 +734,7 @@ sarbp_status sarbp_create(sarbp_ctx **out, int device) {
     // a busy host may preempt for a scheduler slice
     ok = ok && cudaEventCreateWithFlags(&ctx->ev_ext, cudaEventDisableTiming | cudaEventBlockingSync) == cudaSuccess;
     ok = ok && cudaEventCreateWithFlags(&ctx->ev_copy, cudaEventDisableTiming) == cudaSuccess;
+    ok = ok && cudaEventCreateWithFlags(&ctx->ev_scratch, cudaEventDisableTiming) == cudaSuccess;
     ok = ok && cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking) == cudaSuccess;
     ok = ok && cudaMallocHost(reinterpret_cast<void **>(&ctx->ext_host), 8 * sizeof(unsigned long long)) == cudaSuccess;
     if (ok) std::memset(ctx->ext_host, 0, 8 * sizeof(unsigned long long));
@@ -745,6 +766,7 @@ sarbp_status sarbp_destroy(sarbp_ctx *ctx) {
     if (ctx->wkc.ready) cudaEventDestroy(ctx->wkc.ready);
     if (ctx->ceos_ready) cudaEventDestroy(ctx->ceos_ready);
     if (ctx->ev_copy) cudaEventDestroy(ctx->ev_copy);
+    if (ctx->ev_scratch) cudaEventDestroy(ctx->ev_scratch);
     if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
