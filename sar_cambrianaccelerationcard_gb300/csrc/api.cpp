@@ -118,7 +118,7 @@ struct sarbp_ctx {
     cudaStream_t copy_stream = nullptr;      // chunked echo uploads beside range compression
     cudaEvent_t ev_copy = nullptr;
     cudaEvent_t ev_scratch = nullptr;        // end of the last launches that use the back-projection scratch
-    cudaStream_t scratch_stream = nullptr;   // the stream they went to (compared only)
+    bool scratch_used = false;               // recorded at least once
     // Buffers sized by the calls (released by sarbp_trim and sarbp_destroy).
     std::vector<DevBuf *> scratch() {
         std::vector<DevBuf *> v = {&echo,   &spec,  &rc,      &scale,   &apc,     &image,   &partial,
@@ -459,16 +459,17 @@ sarbp_status extremes_device(sarbp_ctx *ctx, const double *apc_dev, int np, cons
 }
 
 // The pulse references, partial images and projection sums live in the context:
-// a call on another stream than the last one's waits for its launches before
-// it overwrites them.
+// every call waits for the last one's launches before it overwrites them (on the
+// same stream they are behind it anyway; streams are not compared by handle, which
+// a per-thread default stream or a destroyed one shares with another).
 sarbp_status scratch_begin(sarbp_ctx *ctx, cudaStream_t s) {
-    if (ctx->scratch_stream && ctx->scratch_stream != s)
+    if (ctx->scratch_used)
         SARBP_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_scratch, 0), "order scratch");
     return SARBP_OK;
 }
 sarbp_status scratch_end(sarbp_ctx *ctx, cudaStream_t s) {
     SARBP_CUDA(ctx, cudaEventRecord(ctx->ev_scratch, s), "order scratch");
-    ctx->scratch_stream = s;
+    ctx->scratch_used = true;
     return SARBP_OK;
 }
 
