@@ -1245,14 +1245,19 @@ size_t bp_smem_bytes(int storage, int win, int chunk) {
 // range 11 ulp (7e-7 relative, kExtR2 is over 5 times that), sine 9e-7 absolute
 // (kExtSin 4 times).  Points whose distance is not well above the rounding of
 // the coordinates, or whose FP32 terms are not ordinary numbers, are always
-// evaluated.  Min and max do not depend on the
-// order, so the bits are the host's.  The last block to finish hands the
-// result to the host (mapped memory, `seq` last) and resets the state for the
-// next call: one launch, no copy.  With the polled result (extremes_wait in
-// api.cpp) a back-projection call of 256 pulses onto 128^2 pixels takes 63 us
-// instead of 129, config 1 as one call 235 instead of 267, a projection of 2048
-// pulses 1.68 ms instead of 1.73.
-constexpr int kExtThreads = 64;
+// evaluated.  They go through a list in shared memory, so that the FP64 chain
+// (about 70 instructions with a square root and a quotient) runs once for a
+// block's few points side by side, not once per lattice column that holds one in
+// some lane.  Min and max do not depend on the order, so the bits are the host's.
+// The last block to finish hands the result to the host (mapped memory, `seq`
+// last) and resets the state for the next call: one launch, no copy.  With the
+// polled result (extremes_wait in api.cpp) a back-projection call of 256 pulses
+// onto 128^2 pixels took 63 us instead of 129 before the list and before small
+// images filled the chip (plan.cpp); with that 49.2, with the list 46.7 (64
+// threads), 44.2 (128) and 42.7 (no reads of the state ahead of its atomics, one
+// system fence).  Threads per block, same call: 32 49.7, 64 47, 96 46, 128 42.7,
+// 192 42.9, 256 47, 288 43.7, 576 45.6.
+constexpr int kExtThreads = 128;
 constexpr float kExtR2 = 4e-6f, kExtSin = 4e-6f;
 struct ExtAxes {
     double len[2];     // |ux|, |uy|
@@ -1272,25 +1277,29 @@ __global__ void __launch_bounds__(kExtThreads)
     __shared__ float Ph[kPts][3], Pl[kPts][3];
     __shared__ float red[4][kExtThreads / 32];
     __shared__ unsigned long long ext[5];
+    __shared__ unsigned short list[kExtThreads * kLattice];  // points to evaluate: thread * 9 + column, cosines wanted
+    __shared__ int count;
     __shared__ bool last;
+    constexpr int kCosX = 1 << 14, kCosY = 1 << 15;
+    static_assert(kExtThreads * kLattice <= kCosX, "list entry");
     const int t = threadIdx.x;
+    const long long i = blockIdx.x * (long long)kExtThreads + t;
+    const int p = (int)(i / kLattice), u = (int)(i - (long long)p * kLattice);
+    bool live = i < (long long)np * kLattice;
+    double a[3] = {0.0, 0.0, 0.0};  // loaded ahead of the lattice's FP64 work
+    if (live)
+        for (int d = 0; d < 3; ++d) a[d] = apc[3 * (size_t)p + d];
     for (int k = t; k < kPts; k += kExtThreads) {
         ext_lattice(g, k / kLattice, k % kLattice, P[k]);
         for (int d = 0; d < 3; ++d) ext_split(P[k][d], Ph[k][d], Pl[k][d]);
     }
+    if (t == 0) count = 0;
     if (t < 5) ext[t] = t == 0 ? (unsigned long long)__double_as_longlong(1e300) : 0ull;
     __syncthreads();
-    const long long i = blockIdx.x * (long long)kExtThreads + t;
-    const int p = (int)(i / kLattice), u = (int)(i - (long long)p * kLattice);
-    double a[3] = {0.0, 0.0, 0.0};
     float ah[3], al[3], size = 0.f;
-    bool live = i < (long long)np * kLattice;
-    if (live) {
-        for (int d = 0; d < 3; ++d) a[d] = apc[3 * (size_t)p + d];
-        if (!isfinite(a[0]) || !isfinite(a[1]) || !isfinite(a[2])) {
-            live = false;
-            ext[4] = 1ull;
-        }
+    if (live && (!isfinite(a[0]) || !isfinite(a[1]) || !isfinite(a[2]))) {
+        live = false;
+        ext[4] = 1ull;
     }
     for (int d = 0; d < 3; ++d) {
         ext_split(a[d], ah[d], al[d]);
@@ -1340,10 +1349,7 @@ __global__ void __launch_bounds__(kExtThreads)
     }
     if (live) {
         const float hi = m[0] * (1.f - kExtR2), lo = m[1] * (1.f + kExtR2), ex = m[2] + kExtSin, ey = m[3] + kExtSin;
-        ExtAcc acc;
-        ext_acc_init(acc);
-        bool any = false;
-#pragma unroll 1
+#pragma unroll
         for (int v = 0; v < kLattice; ++v) {
             float r2, sx, sy, always;
             terms(u * kLattice + v, r2, sx, sy, always);
@@ -1352,33 +1358,41 @@ __global__ void __launch_bounds__(kExtThreads)
             const bool all = !(r2 > always);
             const bool range = all || !(r2 > lo) || !(r2 < hi);
             const bool cos_x = all || !(sx > ex), cos_y = all || !(sy > ey);
-            if (range || cos_x || cos_y) {
-                double r2d, nx, ny;
-                ext_terms(g, P[u * kLattice + v], a, r2d, nx, ny);
-                acc.r2min = fmin(acc.r2min, r2d);
-                acc.r2max = fmax(acc.r2max, r2d);
-                if (r2d > 0) {
-                    if (cos_x && ax.len[0] > 0) ext_cos(acc.cx, nx, r2d, ax.len[0]);
-                    if (cos_y && ax.len[1] > 0) ext_cos(acc.sy, ny, r2d, ax.len[1]);
-                }
-                any = true;
+            if (range || cos_x || cos_y)
+                list[atomicAdd(&count, 1)] = (unsigned short)((t * kLattice + v) | (cos_x ? kCosX : 0) | (cos_y ? kCosY : 0));
+        }
+    }
+    __syncthreads();
+    if (t < count) {
+        ExtAcc acc;
+        ext_acc_init(acc);
+        for (int e = t; e < count; e += kExtThreads) {
+            const int c = list[e], tv = c & (kCosX - 1), tt = tv / kLattice;
+            const long long it = blockIdx.x * (long long)kExtThreads + tt;
+            const long long pe = it / kLattice;
+            const int k = (int)(it - pe * kLattice) * kLattice + tv - tt * kLattice;
+            double ae[3], r2d, nx, ny;
+            for (int d = 0; d < 3; ++d) ae[d] = apc[3 * (size_t)pe + d];
+            ext_terms(g, P[k], ae, r2d, nx, ny);
+            acc.r2min = fmin(acc.r2min, r2d);
+            acc.r2max = fmax(acc.r2max, r2d);
+            if (r2d > 0) {
+                if ((c & kCosX) && ax.len[0] > 0) ext_cos(acc.cx, nx, r2d, ax.len[0]);
+                if ((c & kCosY) && ax.len[1] > 0) ext_cos(acc.sy, ny, r2d, ax.len[1]);
             }
         }
-        if (any) {
-            atomicMin(&ext[0], (unsigned long long)__double_as_longlong(acc.r2min));
-            atomicMax(&ext[1], (unsigned long long)__double_as_longlong(acc.r2max));
-            atomicMax(&ext[2], (unsigned long long)__double_as_longlong(acc.cx.best));
-            atomicMax(&ext[3], (unsigned long long)__double_as_longlong(acc.sy.best));
-        }
+        atomicMin(&ext[0], (unsigned long long)__double_as_longlong(acc.r2min));
+        atomicMax(&ext[1], (unsigned long long)__double_as_longlong(acc.r2max));
+        atomicMax(&ext[2], (unsigned long long)__double_as_longlong(acc.cx.best));
+        atomicMax(&ext[3], (unsigned long long)__double_as_longlong(acc.sy.best));
     }
     __syncthreads();
     // all four quantities are >= 0, where the unsigned order of the bits is the
     // numeric order
     if (t == 0) {
-        volatile unsigned long long *now = state;  // an old value at worst: the atomic decides
-        if (ext[0] < now[0]) atomicMin(&state[0], ext[0]);
+        atomicMin(&state[0], ext[0]);
         for (int k = 1; k < 5; ++k)
-            if (ext[k] > now[k]) atomicMax(&state[k], ext[k]);
+            if (ext[k]) atomicMax(&state[k], ext[k]);
         __threadfence();
         last = atomicAdd(&state[5], 1ull) == gridDim.x - 1;
     }
@@ -1386,12 +1400,11 @@ __global__ void __launch_bounds__(kExtThreads)
     if (last && t < 5) {
         __threadfence();
         result[t] = atomicExch(&state[t], t == 0 ? (unsigned long long)__double_as_longlong(1e300) : 0ull);
-        __threadfence_system();
+        if (t == 0) state[5] = 0ull;
     }
     __syncthreads();
     if (last && t == 0) {
-        state[5] = 0ull;
-        __threadfence_system();
+        __threadfence_system();  // covers what this block wrote before the barrier
         result[5] = seq;
     }
 }

@@ -1,6 +1,5 @@
 // tma.cuh -- shared-memory mbarriers and bulk (TMA) copies for sm_103a, as
-// inline PTX: the staging primitives of the back-projection and the
-// persistent range-compression kernels.
+// inline PTX: the staging primitives of the back-projection kernels.
 #pragma once
 
 #include <cstdint>
