@@ -75,7 +75,7 @@ typedef enum sarbp_mode {
  * half-diagonal use the series form of the phase (about -82 dB against an FP64
  * image); larger ones the linear-term form (per-pixel-step phase increments
  * reduced modulo 2 pi per pulse, FP32 only for the nonlinear remainder: -89 to
- * -113 dB on 0.45-2 m pixels, LINPCT more time); sarbp_bp_plan reports the
+ * -113 dB on 0.45-2 m pixels, 10 to 20% more time); sarbp_bp_plan reports the
  * form (linear_phase). */
 
 /* Storage of range-compressed data. */

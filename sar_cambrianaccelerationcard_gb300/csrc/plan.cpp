@@ -240,7 +240,7 @@ bool plan_bp(int sms, const sarbp_radar &r, const sarbp_rc_view &rc, const BpExt
         // phase form: the series form's FP32 differential range rounds to 2^-24 of
         // n ~ 2 R_T d, a phase error growing with the tile's extent d (about
         // -82 dB below 12 m of half-diagonal, -67 to -74 dB above); the
-        // linear-term form keeps it near -100 dB for ~10% more time
+        // linear-term form keeps it near -100 dB for 10 to 20% more time
         const int force = tune ? tune->linear_phase : 0;
         p.lin = split && (force > 0 || (force == 0 && tile_diag > kLinearPhaseHalfDiag));
         chosen = true;
