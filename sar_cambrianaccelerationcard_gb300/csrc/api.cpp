@@ -170,6 +170,19 @@ sarbp_status cuda_fail(sarbp_ctx *ctx, cudaError_t e, const char *what) {
         if (e_ != cudaSuccess) return cuda_fail(ctx, e_, what); \
     } while (0)
 
+// A host table into device memory, there when this returns: launches on any
+// stream may read it.  (cudaMemcpy goes through the default stream, which the
+// non-blocking streams of the context and its callers do not wait for, and from
+// pageable memory it may return before the device has the data.)
+cudaError_t upload(sarbp_ctx *ctx, void *dst, const void *src, size_t bytes) {
+    const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->copy_stream);
+    return e == cudaSuccess ? cudaStreamSynchronize(ctx->copy_stream) : e;
+}
+cudaError_t clear(sarbp_ctx *ctx, void *dst, size_t bytes) {
+    const cudaError_t e = cudaMemsetAsync(dst, 0, bytes, ctx->copy_stream);
+    return e == cudaSuccess ? cudaStreamSynchronize(ctx->copy_stream) : e;
+}
+
 bool is_device_ptr(const void *p) {
     if (!p) return false;
     cudaPointerAttributes a;
@@ -251,9 +264,8 @@ sarbp_status ensure_tables(sarbp_ctx *ctx, const sarbp_radar *r, const sarbp_rc_
     sarbp::rc_tables_host(*r, lay, g, et);
     SARBP_CUDA(ctx, t.filt.ensure(sizeof(float2) * N), "alloc filter");
     SARBP_CUDA(ctx, t.etab.ensure(sizeof(float2) * et.size()), "alloc phase table");
-    SARBP_CUDA(ctx, cudaMemcpy(t.filt.ptr, g.data(), sizeof(float2) * N, cudaMemcpyHostToDevice), "upload filter");
-    SARBP_CUDA(ctx, cudaMemcpy(t.etab.ptr, et.data(), sizeof(float2) * et.size(), cudaMemcpyHostToDevice),
-               "upload phase table");
+    SARBP_CUDA(ctx, upload(ctx, t.filt.ptr, g.data(), sizeof(float2) * N), "upload filter");
+    SARBP_CUDA(ctx, upload(ctx, t.etab.ptr, et.data(), sizeof(float2) * et.size()), "upload phase table");
     t.valid = true;
     t.nfft = N;
     t.L = L;
@@ -275,7 +287,7 @@ sarbp_status check_errword(sarbp_ctx *ctx) {
     SARBP_CUDA(ctx, cudaMemcpy(&w, ctx->errword.ptr, sizeof w, cudaMemcpyDeviceToHost), "read device check word");
     if (w == 0) return SARBP_OK;
     ctx->last_device_flags = w;
-    SARBP_CUDA(ctx, cudaMemset(ctx->errword.ptr, 0, sizeof(unsigned)), "reset device check word");
+    SARBP_CUDA(ctx, clear(ctx, ctx->errword.ptr, sizeof(unsigned)), "reset device check word");
     if (w & sarbp::kErrDrainTimeout)
         return fail(ctx, SARBP_ERR_TIMEOUT, "a bounded device wait ran out and a copy in flight did not land (0x%x)", w);
     if (w & sarbp::kErrWaitTimeout)
@@ -651,19 +663,15 @@ sarbp_status get_dft(sarbp_ctx *ctx, int n, sarbp::DftPlan &p) {
         sarbp::dft_tables_host(n, etab, chirp, kf, ki);
         slot->n = 0;
         SARBP_CUDA(ctx, slot->etab.ensure(sizeof(float2) * etab.size()), "alloc DFT tables");
-        SARBP_CUDA(ctx, cudaMemcpy(slot->etab.ptr, etab.data(), sizeof(float2) * etab.size(), cudaMemcpyHostToDevice),
-                   "upload DFT tables");
+        SARBP_CUDA(ctx, upload(ctx, slot->etab.ptr, etab.data(), sizeof(float2) * etab.size()), "upload DFT tables");
         slot->m = sarbp::dft_bluestein_size(n);
         if (slot->m) {
             SARBP_CUDA(ctx, slot->chirp.ensure(sizeof(float2) * n), "alloc DFT tables");
             SARBP_CUDA(ctx, slot->kf.ensure(sizeof(float2) * slot->m), "alloc DFT tables");
             SARBP_CUDA(ctx, slot->ki.ensure(sizeof(float2) * slot->m), "alloc DFT tables");
-            SARBP_CUDA(ctx, cudaMemcpy(slot->chirp.ptr, chirp.data(), sizeof(float2) * n, cudaMemcpyHostToDevice),
-                       "upload DFT tables");
-            SARBP_CUDA(ctx, cudaMemcpy(slot->kf.ptr, kf.data(), sizeof(float2) * slot->m, cudaMemcpyHostToDevice),
-                       "upload DFT tables");
-            SARBP_CUDA(ctx, cudaMemcpy(slot->ki.ptr, ki.data(), sizeof(float2) * slot->m, cudaMemcpyHostToDevice),
-                       "upload DFT tables");
+            SARBP_CUDA(ctx, upload(ctx, slot->chirp.ptr, chirp.data(), sizeof(float2) * n), "upload DFT tables");
+            SARBP_CUDA(ctx, upload(ctx, slot->kf.ptr, kf.data(), sizeof(float2) * slot->m), "upload DFT tables");
+            SARBP_CUDA(ctx, upload(ctx, slot->ki.ptr, ki.data(), sizeof(float2) * slot->m), "upload DFT tables");
         }
         slot->n = n;
     }
@@ -742,9 +750,9 @@ sarbp_status sarbp_create(sarbp_ctx **out, int device) {
     unsigned long long ext_state[6];
     sarbp::bp_extremes_state_init(ext_state);
     ok = ok && ctx->ext.ensure(sizeof ext_state) == cudaSuccess &&
-         cudaMemcpy(ctx->ext.ptr, ext_state, sizeof ext_state, cudaMemcpyHostToDevice) == cudaSuccess;
+         upload(ctx, ctx->ext.ptr, ext_state, sizeof ext_state) == cudaSuccess;
     ok = ok && ctx->errword.ensure(sizeof(unsigned)) == cudaSuccess && ctx->power.ensure(sizeof(double)) == cudaSuccess;
-    ok = ok && cudaMemset(ctx->errword.ptr, 0, sizeof(unsigned)) == cudaSuccess;
+    ok = ok && clear(ctx, ctx->errword.ptr, sizeof(unsigned)) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();
         sarbp_destroy(ctx);

@@ -1,0 +1,49 @@
+"""What orders the memory accesses of a context's calls, checked on the CPU.
+
+tests/shim/call_order.cpp links the library's host code with a CUDA runtime of
+its own, which runs nothing and follows what each stream, event and host wait
+orders: two accesses to the same bytes, one of them a write, that nothing orders
+are reported, whatever the timing would have been on a device.  Device-pointer
+calls are asynchronous on the caller's stream, so whatever they share in the
+context has to be ordered by the calls themselves."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "sar_cambrianaccelerationcard_gb300", "csrc")
+
+CALLS = ["autofocus", "bp", "bp_fp16", "bp_host", "ceos", "ceos_host", "dft", "dft2d", "dft_host", "image", "image_fp16",
+         "image_host", "plan", "project", "project_host", "rc", "rc_32768", "rc_fp16", "rc_host", "synth", "synth_host",
+         "wk", "wk_focus", "wk_preprocess"]
+
+
+@pytest.fixture(scope="module")
+def run(tmp_path_factory):
+    cuda = next((d for d in (os.environ.get("CUDA_HOME", ""), "/usr/local/cuda")
+                 if d and os.path.exists(os.path.join(d, "include", "cuda_runtime.h"))), None)
+    if not (shutil.which("g++") and cuda):
+        pytest.skip("needs g++ and the CUDA headers")
+    exe = tmp_path_factory.mktemp("order") / "call_order"
+    subprocess.run(["g++", "-std=c++17", "-O1", "-w", "-I", os.path.join(ROOT, "include"), "-I", CSRC,
+                    "-I", os.path.join(cuda, "include"), os.path.join(ROOT, "tests", "shim", "call_order.cpp"),
+                    os.path.join(CSRC, "api.cpp"), os.path.join(CSRC, "plan.cpp"), "-o", str(exe)], check=True)
+
+    def call(*args):
+        r = subprocess.run([str(exe), *args], capture_output=True, text=True)
+        return r.returncode, r.stdout
+    return call
+
+
+def test_detector_and_call_list(run):
+    assert run("detector")[0] == 0
+    assert run("list")[1].split() == CALLS
+
+
+@pytest.mark.parametrize("name", CALLS)
+def test_first_call_of_a_context(run, name):
+    """Tables and state uploaded for the first call are on the device before its launches read them."""
+    rc, out = run("first", name)
+    assert rc == 0, out
