@@ -18,7 +18,9 @@
  *   - works on caller-owned buffers; pointers may be host or device memory
  *     (detected per call).  With host pointers the call is synchronous; with
  *     device pointers it is asynchronous on `stream` (a cudaStream_t, or NULL
- *     for the context's own stream).
+ *     for the context's own stream).  Calls of one context on different streams
+ *     wait on the device for the earlier calls whose scratch they need; calls
+ *     captured into a graph do not (the caller orders its replays).
  * A context is not thread-safe; use one per host thread.
  *
  * Complex data are interleaved float pairs (layout-compatible with

@@ -92,6 +92,19 @@ struct WkCache {
     cudaEvent_t ready = nullptr;
 };
 
+// What the context's calls share on the device, in groups that are used together.
+// A call on one stream must not touch a group that an earlier call on another
+// stream still uses (ScratchUse); groups are ordered apart, so that range
+// compression of the next aperture still runs beside a back-projection.
+enum Shared {
+    kRows,     // spec, rc, scale
+    kPulses,   // pref, partial, proj
+    kArrays,   // wk0, wk1, wkc
+    kPower,    // power
+    kStaging,  // copies of host arrays and buffers of calls that wait for their result
+    kSharedGroups
+};
+
 }  // namespace
 
 struct sarbp_ctx {
@@ -117,8 +130,8 @@ struct sarbp_ctx {
     cudaEvent_t ev_ext = nullptr;
     cudaStream_t copy_stream = nullptr;      // chunked echo uploads beside range compression
     cudaEvent_t ev_copy = nullptr;
-    cudaEvent_t ev_scratch = nullptr;        // end of the last launches that use the back-projection scratch
-    bool scratch_used = false;               // recorded at least once
+    cudaEvent_t ev_shared[kSharedGroups] = {};  // end of the last call that used each shared group
+    bool shared_used[kSharedGroups] = {};       // recorded at least once
     // Buffers sized by the calls (released by sarbp_trim and sarbp_destroy).
     std::vector<DevBuf *> scratch() {
         std::vector<DevBuf *> v = {&echo,   &spec,  &rc,      &scale,   &apc,     &image,   &partial,
@@ -215,6 +228,49 @@ struct Range {
     Range &operator=(const Range &) = delete;
 };
 
+// One call's use of the shared groups.  begin(), ahead of the first access, makes
+// the stream wait for the last call that used the group, on whatever stream
+// that was (streams are not compared by handle, which a per-thread default stream
+// or a destroyed one shares with another); the end is marked behind everything the
+// call queued, on error returns too.  While the stream is being captured neither
+// is done (a capture cannot wait for work outside it): whoever replays the graph
+// orders it against the context's other calls.
+class ScratchUse {
+  public:
+    ScratchUse(sarbp_ctx *ctx, cudaStream_t s) : ctx_(ctx), s_(s) {
+        cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s, &c) != cudaSuccess) cudaGetLastError();
+        capturing_ = c != cudaStreamCaptureStatusNone;
+    }
+    ScratchUse(const ScratchUse &) = delete;
+    ScratchUse &operator=(const ScratchUse &) = delete;
+    sarbp_status begin(Shared group) {
+        if (capturing_ || begun_[group]) return SARBP_OK;
+        if (ctx_->shared_used[group])
+            SARBP_CUDA(ctx_, cudaStreamWaitEvent(s_, ctx_->ev_shared[group], 0), "order shared scratch");
+        begun_[group] = true;
+        return SARBP_OK;
+    }
+    ~ScratchUse() {
+        for (int k = 0; k < kSharedGroups; ++k) {
+            if (!begun_[k]) continue;
+            if (cudaEventRecord(ctx_->ev_shared[k], s_) == cudaSuccess) ctx_->shared_used[k] = true;
+            else cudaGetLastError();
+        }
+    }
+
+  private:
+    sarbp_ctx *ctx_;
+    cudaStream_t s_;
+    bool capturing_ = false;
+    bool begun_[kSharedGroups] = {};
+};
+#define SARBP_BEGIN(use, group)                               \
+    do {                                                      \
+        const sarbp_status st_ = (use).begin(group);          \
+        if (st_ != SARBP_OK) return st_;                      \
+    } while (0)
+
 bool is_pow2(long long n) { return n > 0 && (n & (n - 1)) == 0; }
 
 long long next_pow2(long long n) {
@@ -310,12 +366,13 @@ sarbp_status finish(sarbp_ctx *ctx, cudaStream_t s, bool sync) {
 
 // Range compression of a device-resident echo into a device rc buffer.
 sarbp_status rc_device(sarbp_ctx *ctx, const sarbp_radar *r, const sarbp_rc_layout &lay, const float2 *echo,
-                       int np, int ns, int storage, void *rc_out, float *scale_out, cudaStream_t s,
+                       int np, int ns, int storage, void *rc_out, float *scale_out, cudaStream_t s, ScratchUse &use,
                        bool record_events = true) {
     Range range("sarbp: range compression");
     if (!sarbp::rc_size_supported(lay.nfft))
         return fail(ctx, SARBP_ERR_UNSUPPORTED, "range FFT size %d not supported (max 32768: ns + tp*fs - 1 <= 32768)",
                     lay.nfft);
+    SARBP_BEGIN(use, kRows);
     sarbp_status st = ensure_tables(ctx, r, lay);
     if (st != SARBP_OK) return st;
     const size_t row = sizeof(float2) * (size_t)lay.nfft;
@@ -360,7 +417,8 @@ sarbp_status rc_device(sarbp_ctx *ctx, const sarbp_radar *r, const sarbp_rc_layo
 // context's echo buffer).
 sarbp_status rc_host_echo_enqueue(sarbp_ctx *ctx, const sarbp_radar *r, const sarbp_rc_layout &lay,
                                   const sarbp_complex64 *echo, int np, int ns, int storage, void *rc_out,
-                                  float *scale_out, cudaStream_t s) {
+                                  float *scale_out, cudaStream_t s, ScratchUse &use) {
+    SARBP_BEGIN(use, kStaging);
     SARBP_CUDA(ctx, ctx->echo.ensure(sizeof(float2) * (size_t)np * ns), "alloc echo");
     float2 *d_echo = ctx->echo.as<float2>();
     const size_t row = sizeof(float2) * (size_t)ns;
@@ -384,7 +442,7 @@ sarbp_status rc_host_echo_enqueue(sarbp_ctx *ctx, const sarbp_radar *r, const sa
         SARBP_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_copy, 0), "upload echo");
         sarbp_status st = rc_device(ctx, r, lay, d_echo + (size_t)p0 * ns, n, ns, storage,
                                     static_cast<char *>(rc_out) + (size_t)p0 * lay.nbins * esize,
-                                    scale_out ? scale_out + p0 : nullptr, s, false);
+                                    scale_out ? scale_out + p0 : nullptr, s, use, false);
         if (st != SARBP_OK) return st;
     }
     cudaEventRecord(ctx->ev[1], s);
@@ -400,9 +458,10 @@ void drain_uploads(sarbp_ctx *ctx) {
 }
 
 sarbp_status rc_host_echo(sarbp_ctx *ctx, const sarbp_radar *r, const sarbp_rc_layout &lay, const sarbp_complex64 *echo,
-                          int np, int ns, int storage, void *rc_out, float *scale_out, cudaStream_t s) {
+                          int np, int ns, int storage, void *rc_out, float *scale_out, cudaStream_t s,
+                          ScratchUse &use) {
     Range range("sarbp: chunked echo upload + range compression");
-    const sarbp_status st = rc_host_echo_enqueue(ctx, r, lay, echo, np, ns, storage, rc_out, scale_out, s);
+    const sarbp_status st = rc_host_echo_enqueue(ctx, r, lay, echo, np, ns, storage, rc_out, scale_out, s, use);
     if (st != SARBP_OK) drain_uploads(ctx);
     return st;
 }
@@ -470,25 +529,11 @@ sarbp_status extremes_device(sarbp_ctx *ctx, const double *apc_dev, int np, cons
     return st != SARBP_OK ? st : extremes_wait(ctx, e);
 }
 
-// The pulse references, partial images and projection sums live in the context:
-// every call waits for the last one's launches before it overwrites them (on the
-// same stream they are behind it anyway; streams are not compared by handle, which
-// a per-thread default stream or a destroyed one shares with another).
-sarbp_status scratch_begin(sarbp_ctx *ctx, cudaStream_t s) {
-    if (ctx->scratch_used)
-        SARBP_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev_scratch, 0), "order scratch");
-    return SARBP_OK;
-}
-sarbp_status scratch_end(sarbp_ctx *ctx, cudaStream_t s) {
-    SARBP_CUDA(ctx, cudaEventRecord(ctx->ev_scratch, s), "order scratch");
-    ctx->scratch_used = true;
-    return SARBP_OK;
-}
-
 // Back-projection of device-resident rc + apc into a device image.
 sarbp_status bp_device(sarbp_ctx *ctx, const sarbp_radar *r, const sarbp_rc_view &rc, const double *apc_dev,
                        const sarbp::BpExtremes &ex, const sarbp_grid *g, int mode, float2 *image, int accumulate,
-                       cudaStream_t s, const double *dr_dev = nullptr, const double *dph_dev = nullptr) {
+                       cudaStream_t s, ScratchUse &use, const double *dr_dev = nullptr,
+                       const double *dph_dev = nullptr) {
     Range range("sarbp: back-projection");
     const int np = rc.np;
     if (g->nx == 0 || g->ny == 0) return SARBP_OK;
@@ -520,21 +565,21 @@ sarbp_status bp_device(sarbp_ctx *ctx, const sarbp_radar *r, const sarbp_rc_view
         p.partial = ctx->partial.as<float2>();
     }
     int launches = 0;
-    sarbp_status st = scratch_begin(ctx, s);
-    if (st != SARBP_OK) return st;
+    SARBP_BEGIN(use, kPulses);
     cudaEventRecord(ctx->ev[2], s);
     SARBP_CUDA(ctx, sarbp::launch_bp(p, s, &launches), "back-projection launch");
     cudaEventRecord(ctx->ev[3], s);
     ctx->timed_bp = true;
     ctx->launches += launches;
-    return scratch_end(ctx, s);
+    return SARBP_OK;
 }
 
 // Weighted projection of device-resident rc + apc against a device weight
 // image into out[np] (device, complex128).
 sarbp_status project_device(sarbp_ctx *ctx, const sarbp_radar *r, const sarbp_rc_view &rc, const double *apc_dev,
                             const sarbp::BpExtremes &ex, const sarbp_grid *g, int mode, const float2 *weight,
-                            double2 *out, cudaStream_t s, const double *dr_dev, const double *dph_dev) {
+                            double2 *out, cudaStream_t s, ScratchUse &use, const double *dr_dev,
+                            const double *dph_dev) {
     Range range("sarbp: weighted projection");
     const int np = rc.np;
     if (np == 0) return SARBP_OK;
@@ -558,11 +603,10 @@ sarbp_status project_device(sarbp_ctx *ctx, const sarbp_radar *r, const sarbp_rc
     SARBP_CUDA(ctx, ctx->proj.ensure(sizeof(float2) * sarbp::bp_tiles(p) * (size_t)np), "alloc projection scratch");
     p.proj = ctx->proj.as<float2>();
     int launches = 0;
-    sarbp_status st = scratch_begin(ctx, s);
-    if (st != SARBP_OK) return st;
+    SARBP_BEGIN(use, kPulses);
     SARBP_CUDA(ctx, sarbp::launch_project(p, out, s, &launches), "projection launch");
     ctx->launches += launches;
-    return scratch_end(ctx, s);
+    return SARBP_OK;
 }
 
 // Device-side inputs of a back-projection-type call (uploads of host arrays
@@ -577,7 +621,7 @@ struct BpInputs {
 
 sarbp_status stage_bp_inputs(sarbp_ctx *ctx, const sarbp_radar *radar, const sarbp_rc_view *rc, const double *apc,
                              const sarbp_grid *grid, int32_t mode, const sarbp_pulse_corr *corr, cudaStream_t s,
-                             BpInputs &in) {
+                             ScratchUse &use, BpInputs &in) {
     sarbp_status st = check_radar(ctx, radar);
     if (st != SARBP_OK) return st;
     if (!rc) return fail(ctx, SARBP_ERR_INVALID_ARGUMENT, "rc view is null");
@@ -603,6 +647,7 @@ sarbp_status stage_bp_inputs(sarbp_ctx *ctx, const sarbp_radar *radar, const sar
     if (np == 0) return SARBP_OK;
     // APC on the device for the kernel; the planner's extremes are reduced there
     if (!is_device_ptr(apc)) {
+        SARBP_BEGIN(use, kStaging);
         SARBP_CUDA(ctx, ctx->apc.ensure(sizeof(double) * 3 * np), "alloc apc");
         SARBP_CUDA(ctx, cudaMemcpyAsync(ctx->apc.ptr, apc, sizeof(double) * 3 * np, cudaMemcpyHostToDevice, s),
                    "upload apc");
@@ -612,6 +657,7 @@ sarbp_status stage_bp_inputs(sarbp_ctx *ctx, const sarbp_radar *radar, const sar
     st = extremes_device(ctx, in.apc_dev, np, grid, s, in.ex);
     if (st != SARBP_OK) return st;
     if (!is_device_ptr(rc->data)) {
+        SARBP_BEGIN(use, kRows);
         SARBP_CUDA(ctx, ctx->rc.ensure(esize * (size_t)np * rc->nbins), "alloc rc");
         SARBP_CUDA(ctx, cudaMemcpyAsync(ctx->rc.ptr, rc->data, esize * (size_t)np * rc->nbins, cudaMemcpyHostToDevice, s),
                    "upload rc");
@@ -619,6 +665,7 @@ sarbp_status stage_bp_inputs(sarbp_ctx *ctx, const sarbp_radar *radar, const sar
         in.any_host = true;
     }
     if (rc->storage == SARBP_STORE_C32H && !is_device_ptr(rc->scale)) {
+        SARBP_BEGIN(use, kRows);
         SARBP_CUDA(ctx, ctx->scale.ensure(sizeof(float) * np), "alloc scale");
         SARBP_CUDA(ctx, cudaMemcpyAsync(ctx->scale.ptr, rc->scale, sizeof(float) * np, cudaMemcpyHostToDevice, s),
                    "upload scale");
@@ -626,6 +673,7 @@ sarbp_status stage_bp_inputs(sarbp_ctx *ctx, const sarbp_radar *radar, const sar
         in.any_host = true;
     }
     if (corr && (corr->drange || corr->dphase)) {
+        SARBP_BEGIN(use, kStaging);
         SARBP_CUDA(ctx, ctx->corr.ensure(sizeof(double) * 2 * (size_t)np), "alloc corrections");
         const double *src[2] = {corr->drange, corr->dphase};
         const double **dst[2] = {&in.dr_dev, &in.dph_dev};
@@ -743,7 +791,7 @@ sarbp_status sarbp_create(sarbp_ctx **out, int device) {
     // a busy host may preempt for a scheduler slice
     ok = ok && cudaEventCreateWithFlags(&ctx->ev_ext, cudaEventDisableTiming | cudaEventBlockingSync) == cudaSuccess;
     ok = ok && cudaEventCreateWithFlags(&ctx->ev_copy, cudaEventDisableTiming) == cudaSuccess;
-    ok = ok && cudaEventCreateWithFlags(&ctx->ev_scratch, cudaEventDisableTiming) == cudaSuccess;
+    for (cudaEvent_t &e : ctx->ev_shared) ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
     ok = ok && cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking) == cudaSuccess;
     ok = ok && cudaMallocHost(reinterpret_cast<void **>(&ctx->ext_host), 8 * sizeof(unsigned long long)) == cudaSuccess;
     if (ok) std::memset(ctx->ext_host, 0, 8 * sizeof(unsigned long long));
@@ -775,7 +823,8 @@ sarbp_status sarbp_destroy(sarbp_ctx *ctx) {
     if (ctx->wkc.ready) cudaEventDestroy(ctx->wkc.ready);
     if (ctx->ceos_ready) cudaEventDestroy(ctx->ceos_ready);
     if (ctx->ev_copy) cudaEventDestroy(ctx->ev_copy);
-    if (ctx->ev_scratch) cudaEventDestroy(ctx->ev_scratch);
+    for (cudaEvent_t e : ctx->ev_shared)
+        if (e) cudaEventDestroy(e);
     if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
@@ -832,6 +881,8 @@ sarbp_status sarbp_range_compress(sarbp_ctx *ctx, const sarbp_radar *radar, cons
     if (storage == SARBP_STORE_C32H && !rc_scale_out)
         return fail(ctx, SARBP_ERR_INVALID_ARGUMENT, "fp16 storage needs rc_scale_out");
     cudaStream_t s = pick_stream(ctx, stream);
+    ScratchUse use(ctx, s);
+    SARBP_BEGIN(use, kRows);
     const size_t esize = storage == SARBP_STORE_C64 ? 8 : 4;
     const bool dev_in = is_device_ptr(echo), dev_out = is_device_ptr(rc_out);
     const bool dev_sc = storage == SARBP_STORE_C64 || is_device_ptr(rc_scale_out);
@@ -847,8 +898,8 @@ sarbp_status sarbp_range_compress(sarbp_ctx *ctx, const sarbp_radar *radar, cons
         d_scale = ctx->scale.as<float>();
     }
     ctx->timed_bp = false;
-    st = dev_in ? rc_device(ctx, radar, lay, d_echo, np, ns, storage, d_rc, storage == SARBP_STORE_C32H ? d_scale : nullptr, s)
-                : rc_host_echo(ctx, radar, lay, echo, np, ns, storage, d_rc, storage == SARBP_STORE_C32H ? d_scale : nullptr, s);
+    st = dev_in ? rc_device(ctx, radar, lay, d_echo, np, ns, storage, d_rc, storage == SARBP_STORE_C32H ? d_scale : nullptr, s, use)
+                : rc_host_echo(ctx, radar, lay, echo, np, ns, storage, d_rc, storage == SARBP_STORE_C32H ? d_scale : nullptr, s, use);
     if (st != SARBP_OK) return st;
     if (!dev_out)
         SARBP_CUDA(ctx, cudaMemcpyAsync(rc_out, d_rc, esize * (size_t)np * lay.nbins, cudaMemcpyDeviceToHost, s),
@@ -869,8 +920,9 @@ sarbp_status sarbp_backproject_ex(sarbp_ctx *ctx, const sarbp_radar *radar, cons
     cudaStream_t s = pick_stream(ctx, stream);
     if (grid && (size_t)grid->nx * grid->ny > 0 && !image)
         return fail(ctx, SARBP_ERR_INVALID_ARGUMENT, "image is null");
+    ScratchUse use(ctx, s);
     BpInputs in;
-    sarbp_status st = stage_bp_inputs(ctx, radar, rc, apc, grid, mode, corr, s, in);
+    sarbp_status st = stage_bp_inputs(ctx, radar, rc, apc, grid, mode, corr, s, use, in);
     if (st != SARBP_OK) return st;
     const size_t npix = (size_t)grid->nx * grid->ny;
     if (npix == 0) return SARBP_OK;
@@ -878,6 +930,7 @@ sarbp_status sarbp_backproject_ex(sarbp_ctx *ctx, const sarbp_radar *radar, cons
     const bool dev_img = is_device_ptr(image);
     bool any_host = in.any_host;
     if (!dev_img) {
+        SARBP_BEGIN(use, kStaging);
         SARBP_CUDA(ctx, ctx->image.ensure(sizeof(float2) * npix), "alloc image");
         d_img = ctx->image.as<float2>();
         if (accumulate)
@@ -885,7 +938,7 @@ sarbp_status sarbp_backproject_ex(sarbp_ctx *ctx, const sarbp_radar *radar, cons
         any_host = true;
     }
     ctx->timed_rc = false;
-    st = bp_device(ctx, radar, in.v, in.apc_dev, in.ex, grid, mode, d_img, accumulate, s, in.dr_dev, in.dph_dev);
+    st = bp_device(ctx, radar, in.v, in.apc_dev, in.ex, grid, mode, d_img, accumulate, s, use, in.dr_dev, in.dph_dev);
     if (st != SARBP_OK) return st;
     if (!dev_img)
         SARBP_CUDA(ctx, cudaMemcpyAsync(image, d_img, sizeof(float2) * npix, cudaMemcpyDeviceToHost, s), "download image");
@@ -923,8 +976,10 @@ sarbp_status sarbp_bp_plan(sarbp_ctx *ctx, const sarbp_radar *radar, const sarbp
         sarbp::bp_extremes_host(apc, np, *grid, ex);
         if (ex.nonfinite) return fail(ctx, SARBP_ERR_INVALID_ARGUMENT, "apc must be finite");
     } else {
+        ScratchUse use(ctx, ctx->stream);
         const double *apc_dev = apc;
         if (!is_device_ptr(apc)) {
+            SARBP_BEGIN(use, kStaging);
             SARBP_CUDA(ctx, ctx->apc.ensure(sizeof(double) * 3 * np), "alloc apc");
             SARBP_CUDA(ctx, cudaMemcpyAsync(ctx->apc.ptr, apc, sizeof(double) * 3 * np, cudaMemcpyHostToDevice, ctx->stream),
                        "upload apc");
@@ -970,8 +1025,9 @@ sarbp_status sarbp_project_weighted(sarbp_ctx *ctx, const sarbp_radar *radar, co
     if (mode != SARBP_MODE_SPLIT && mode != SARBP_MODE_FP16STORE)
         return fail(ctx, SARBP_ERR_UNSUPPORTED, "weighted projection runs in SPLIT or FP16STORE mode");
     cudaStream_t s = pick_stream(ctx, stream);
+    ScratchUse use(ctx, s);
     BpInputs in;
-    sarbp_status st = stage_bp_inputs(ctx, radar, rc, apc, grid, mode, corr, s, in);
+    sarbp_status st = stage_bp_inputs(ctx, radar, rc, apc, grid, mode, corr, s, use, in);
     if (st != SARBP_OK) return st;
     const int np = rc->np;
     if (np == 0) return SARBP_OK;
@@ -981,6 +1037,7 @@ sarbp_status sarbp_project_weighted(sarbp_ctx *ctx, const sarbp_radar *radar, co
     double2 *d_out = reinterpret_cast<double2 *>(out);
     const bool dev_out = is_device_ptr(out);
     if (!dev_out) {
+        SARBP_BEGIN(use, kStaging);
         SARBP_CUDA(ctx, ctx->projout.ensure(sizeof(double2) * np), "alloc projection output");
         d_out = ctx->projout.as<double2>();
         any_host = true;
@@ -991,13 +1048,14 @@ sarbp_status sarbp_project_weighted(sarbp_ctx *ctx, const sarbp_radar *radar, co
         if (!weight) return fail(ctx, SARBP_ERR_INVALID_ARGUMENT, "weight is null");
         const float2 *d_w = reinterpret_cast<const float2 *>(weight);
         if (!is_device_ptr(weight)) {
+            SARBP_BEGIN(use, kStaging);
             SARBP_CUDA(ctx, ctx->weight.ensure(sizeof(float2) * npix), "alloc weight");
             SARBP_CUDA(ctx, cudaMemcpyAsync(ctx->weight.ptr, weight, sizeof(float2) * npix, cudaMemcpyHostToDevice, s),
                        "upload weight");
             d_w = ctx->weight.as<float2>();
             any_host = true;
         }
-        st = project_device(ctx, radar, in.v, in.apc_dev, in.ex, grid, mode, d_w, d_out, s, in.dr_dev,
+        st = project_device(ctx, radar, in.v, in.apc_dev, in.ex, grid, mode, d_w, d_out, s, use, in.dr_dev,
                             in.dph_dev);
         if (st != SARBP_OK) return st;
     }
@@ -1021,9 +1079,11 @@ sarbp_status sarbp_autofocus(sarbp_ctx *ctx, const sarbp_radar *radar, const sar
         return fail(ctx, SARBP_ERR_INVALID_ARGUMENT, "dphase, drange and sharpness are host arrays");
     cudaStream_t s = pick_stream(ctx, stream);
     sarbp_pulse_corr c0{drange, nullptr};
+    ScratchUse use(ctx, s);
     BpInputs in;
-    sarbp_status st = stage_bp_inputs(ctx, radar, rc, apc, grid, mode, &c0, s, in);
+    sarbp_status st = stage_bp_inputs(ctx, radar, rc, apc, grid, mode, &c0, s, use, in);
     if (st != SARBP_OK) return st;
+    SARBP_BEGIN(use, kStaging);
     const int np = rc->np;
     const size_t npix = (size_t)grid->nx * grid->ny;
     if (np == 0 || npix == 0) return finish(ctx, s, true);
@@ -1049,7 +1109,7 @@ sarbp_status sarbp_autofocus(sarbp_ctx *ctx, const sarbp_radar *radar, const sar
     float2 *d_w = ctx->weight.as<float2>();
     for (int it = 0; it <= iterations; ++it) {
         SARBP_CUDA(ctx, cudaMemcpyAsync(d_ph, ph.data(), sizeof(double) * np, cudaMemcpyHostToDevice, s), "upload phases");
-        st = bp_device(ctx, radar, in.v, in.apc_dev, in.ex, grid, mode, d_img, 0, s, in.dr_dev, d_ph);
+        st = bp_device(ctx, radar, in.v, in.apc_dev, in.ex, grid, mode, d_img, 0, s, use, in.dr_dev, d_ph);
         if (st != SARBP_OK) return st;
         const bool last = it == iterations;
         SARBP_CUDA(ctx, sarbp::launch_sharpness_weight(d_img, npix, last ? nullptr : d_w, ctx->sharp.as<double>(), s),
@@ -1057,7 +1117,7 @@ sarbp_status sarbp_autofocus(sarbp_ctx *ctx, const sarbp_radar *radar, const sar
         ctx->launches += 1;
         if (!last) {
             st = project_device(ctx, radar, in.v, in.apc_dev, in.ex, grid, mode, d_w, ctx->projout.as<double2>(),
-                                s, in.dr_dev, d_ph);
+                                s, use, in.dr_dev, d_ph);
             if (st != SARBP_OK) return st;
             SARBP_CUDA(ctx, cudaMemcpyAsync(cp.data(), ctx->projout.ptr, sizeof(double2) * np, cudaMemcpyDeviceToHost, s),
                        "download projection");
@@ -1108,10 +1168,12 @@ sarbp_status sarbp_dft(sarbp_ctx *ctx, sarbp_complex64 *data, int32_t rows, int3
     sarbp_status st = get_dft(ctx, n, p);
     if (st != SARBP_OK) return st;
     cudaStream_t s = pick_stream(ctx, stream);
+    ScratchUse use(ctx, s);
     const size_t bytes = sizeof(float2) * (size_t)rows * n;
     float2 *d = reinterpret_cast<float2 *>(data);
     const bool dev = is_device_ptr(data);
     if (!dev) {
+        SARBP_BEGIN(use, kArrays);
         SARBP_CUDA(ctx, ctx->wk0.ensure(bytes), "alloc DFT buffer");
         d = ctx->wk0.as<float2>();
         SARBP_CUDA(ctx, cudaMemcpyAsync(d, data, bytes, cudaMemcpyHostToDevice, s), "upload DFT rows");
@@ -1139,10 +1201,12 @@ sarbp_status sarbp_dft2d(sarbp_ctx *ctx, sarbp_complex64 *data, int32_t na, int3
     if (na > 1 && (st = get_dft(ctx, na, pa)) != SARBP_OK) return st;
     if (nr > 1 && na > 1 && na != nr && (st = get_dft(ctx, nr, pr)) != SARBP_OK) return st;  // both still cached
     cudaStream_t s = pick_stream(ctx, stream);
+    ScratchUse use(ctx, s);
     const size_t bytes = sizeof(float2) * (size_t)na * nr;
     float2 *d = reinterpret_cast<float2 *>(data);
     const bool dev = is_device_ptr(data);
     if (!dev) {
+        SARBP_BEGIN(use, kArrays);
         SARBP_CUDA(ctx, ctx->wk0.ensure(bytes), "alloc DFT buffer");
         d = ctx->wk0.as<float2>();
         SARBP_CUDA(ctx, cudaMemcpyAsync(d, data, bytes, cudaMemcpyHostToDevice, s), "upload DFT array");
@@ -1158,6 +1222,7 @@ sarbp_status sarbp_dft2d(sarbp_ctx *ctx, sarbp_complex64 *data, int32_t na, int3
             SARBP_CUDA(ctx, sarbp::launch_dft_cols(pa, d, d, nr, inv, sc, s), "column DFT");
             ctx->launches += 1;
         } else {
+            SARBP_BEGIN(use, kArrays);
             SARBP_CUDA(ctx, ctx->wk1.ensure(bytes), "alloc transpose buffer");
             float2 *t = ctx->wk1.as<float2>();
             SARBP_CUDA(ctx, sarbp::launch_transpose(d, t, na, nr, s), "transpose");
@@ -1309,6 +1374,9 @@ sarbp_status sarbp_wk_image(sarbp_ctx *ctx, const sarbp_wk_params *w, const sarb
     st = get_dft(ctx, NA, pa_plan);
     if (st != SARBP_OK) return st;
     cudaStream_t s = pick_stream(ctx, stream);
+    ScratchUse use(ctx, s);
+    SARBP_BEGIN(use, kArrays);
+    SARBP_BEGIN(use, kStaging);
     WkTables tb;
     st = wk_tables(ctx, w, NA, NR, s, tb);
     if (st != SARBP_OK) return st;
@@ -1384,6 +1452,9 @@ sarbp_status sarbp_wk_preprocess(sarbp_ctx *ctx, const sarbp_wk_params *w, const
     int pa, pr;
     wk_pads(na, nr, &pa, &pr);
     cudaStream_t s = pick_stream(ctx, stream);
+    ScratchUse use(ctx, s);
+    SARBP_BEGIN(use, kArrays);
+    SARBP_BEGIN(use, kStaging);
     WkTables tb;
     st = wk_tables(ctx, w, NA, NR, s, tb);
     if (st != SARBP_OK) return st;
@@ -1420,6 +1491,9 @@ sarbp_status sarbp_wk_focus(sarbp_ctx *ctx, const sarbp_wk_params *w, const sarb
     if (sarbp::wk_stolt_smem(nr_pad) > (size_t)(227u << 10))
         return fail(ctx, SARBP_ERR_UNSUPPORTED, "range size %d too large for the Stolt stage", nr_pad);
     cudaStream_t s = pick_stream(ctx, stream);
+    ScratchUse use(ctx, s);
+    SARBP_BEGIN(use, kArrays);
+    SARBP_BEGIN(use, kStaging);
     WkTables tb;
     st = wk_tables(ctx, w, na_pad, nr_pad, s, tb);
     if (st != SARBP_OK) return st;
@@ -1482,12 +1556,14 @@ sarbp_status sarbp_ceos_decode(sarbp_ctx *ctx, const uint8_t *raw, uint64_t raw_
         return fail(ctx, SARBP_ERR_INVALID_ARGUMENT, "raw data end at byte %llu, the lines need %lld",
                     (unsigned long long)raw_bytes, hi);
     cudaStream_t s = pick_stream(ctx, stream);
+    ScratchUse use(ctx, s);
     bool any_host = false;
     const unsigned char *d_raw;
     if (is_device_ptr(raw)) {
         d_raw = reinterpret_cast<const unsigned char *>(raw);
         g.raw_offset = -(long long)l->file_header;
     } else {
+        SARBP_BEGIN(use, kStaging);
         SARBP_CUDA(ctx, ctx->echo.ensure((size_t)(hi - lo)), "alloc raw buffer");
         SARBP_CUDA(ctx, cudaMemcpyAsync(ctx->echo.ptr, raw + lo, (size_t)(hi - lo), cudaMemcpyHostToDevice, s),
                    "upload raw blocks");
@@ -1518,6 +1594,7 @@ sarbp_status sarbp_ceos_decode(sarbp_ctx *ctx, const uint8_t *raw, uint64_t raw_
     const size_t out_bytes = sizeof(float2) * (size_t)nlines * ncells;
     const bool dev_echo = is_device_ptr(echo);
     if (!dev_echo) {
+        SARBP_BEGIN(use, kArrays);
         SARBP_CUDA(ctx, ctx->wk0.ensure(out_bytes), "alloc echo");
         d_echo = ctx->wk0.as<float2>();
         any_host = true;
@@ -1527,6 +1604,7 @@ sarbp_status sarbp_ceos_decode(sarbp_ctx *ctx, const uint8_t *raw, uint64_t raw_
         if (is_device_ptr(agc_db)) {
             d_agc = reinterpret_cast<short *>(agc_db);
         } else {
+            SARBP_BEGIN(use, kStaging);
             SARBP_CUDA(ctx, ctx->sharp.ensure(sizeof(short) * nlines), "alloc agc");
             d_agc = ctx->sharp.as<short>();
             any_host = true;
@@ -1561,6 +1639,7 @@ sarbp_status sarbp_image(sarbp_ctx *ctx, const sarbp_radar *radar, const sarbp_c
     if (!image) return fail(ctx, SARBP_ERR_INVALID_ARGUMENT, "image is null");
     if (np > 0 && (!echo || !apc)) return fail(ctx, SARBP_ERR_INVALID_ARGUMENT, "echo and apc must be non-null");
     cudaStream_t s = pick_stream(ctx, stream);
+    ScratchUse use(ctx, s);
     const int storage = mode == SARBP_MODE_FP16STORE ? SARBP_STORE_C32H : SARBP_STORE_C64;
     const size_t esize = storage == SARBP_STORE_C64 ? 8 : 4;
     bool any_host = false;
@@ -1571,6 +1650,7 @@ sarbp_status sarbp_image(sarbp_ctx *ctx, const sarbp_radar *radar, const sarbp_c
     sarbp::BpExtremes ex{};
     if (np > 0) {
         if (!is_device_ptr(apc)) {
+            SARBP_BEGIN(use, kStaging);
             SARBP_CUDA(ctx, ctx->apc.ensure(sizeof(double) * 3 * np), "alloc apc");
             SARBP_CUDA(ctx, cudaMemcpyAsync(ctx->apc.ptr, apc, sizeof(double) * 3 * np, cudaMemcpyHostToDevice, s),
                        "upload apc");
@@ -1590,6 +1670,7 @@ sarbp_status sarbp_image(sarbp_ctx *ctx, const sarbp_radar *radar, const sarbp_c
         d_img = mapped_img;
         any_host = true;
     } else if (!dev_img) {
+        SARBP_BEGIN(use, kStaging);
         SARBP_CUDA(ctx, ctx->image.ensure(sizeof(float2) * npix), "alloc image");
         d_img = ctx->image.as<float2>();
         any_host = true;
@@ -1603,12 +1684,13 @@ sarbp_status sarbp_image(sarbp_ctx *ctx, const sarbp_radar *radar, const sarbp_c
     v.t0_bins = lay.t0_bins;
     v.bin_rate = lay.bin_rate;
     if (np > 0) {
+        SARBP_BEGIN(use, kRows);
         SARBP_CUDA(ctx, ctx->rc.ensure(esize * (size_t)np * lay.nbins), "alloc rc");
         if (storage == SARBP_STORE_C32H) SARBP_CUDA(ctx, ctx->scale.ensure(sizeof(float) * np), "alloc scale");
         float *d_scale = storage == SARBP_STORE_C32H ? ctx->scale.as<float>() : nullptr;
-        st = host_echo ? rc_host_echo(ctx, radar, lay, echo, np, ns, storage, ctx->rc.ptr, d_scale, s)
+        st = host_echo ? rc_host_echo(ctx, radar, lay, echo, np, ns, storage, ctx->rc.ptr, d_scale, s, use)
                        : rc_device(ctx, radar, lay, reinterpret_cast<const float2 *>(echo), np, ns, storage, ctx->rc.ptr,
-                                   d_scale, s);
+                                   d_scale, s, use);
         if (st != SARBP_OK) return st;
         v.data = ctx->rc.ptr;
         v.scale = storage == SARBP_STORE_C32H ? ctx->scale.as<float>() : nullptr;
@@ -1618,7 +1700,7 @@ sarbp_status sarbp_image(sarbp_ctx *ctx, const sarbp_radar *radar, const sarbp_c
             return st;
         }
     }
-    st = bp_device(ctx, radar, v, apc_dev, ex, grid, mode, d_img, 0, s);
+    st = bp_device(ctx, radar, v, apc_dev, ex, grid, mode, d_img, 0, s, use);
     if (st != SARBP_OK) {
         if (host_echo) drain_uploads(ctx);
         return st;
@@ -1646,9 +1728,12 @@ sarbp_status sarbp_synthesize_echo(sarbp_ctx *ctx, const sarbp_radar *radar, con
     if (np == 0) return SARBP_OK;
     if (!apc || !echo_out || (nt > 0 && !targets)) return fail(ctx, SARBP_ERR_INVALID_ARGUMENT, "null pointer");
     cudaStream_t s = pick_stream(ctx, stream);
+    ScratchUse use(ctx, s);
+    SARBP_BEGIN(use, kPower);
     bool any_host = false;
     const double *d_apc = apc;
     if (!is_device_ptr(apc)) {
+        SARBP_BEGIN(use, kStaging);
         SARBP_CUDA(ctx, ctx->apc.ensure(sizeof(double) * 3 * np), "alloc apc");
         SARBP_CUDA(ctx, cudaMemcpyAsync(ctx->apc.ptr, apc, sizeof(double) * 3 * np, cudaMemcpyHostToDevice, s), "upload apc");
         d_apc = ctx->apc.as<double>();
@@ -1656,6 +1741,7 @@ sarbp_status sarbp_synthesize_echo(sarbp_ctx *ctx, const sarbp_radar *radar, con
     }
     const sarbp_target *d_tg = targets;
     if (nt > 0 && !is_device_ptr(targets)) {
+        SARBP_BEGIN(use, kStaging);
         SARBP_CUDA(ctx, ctx->targets.ensure(sizeof(sarbp_target) * nt), "alloc targets");
         SARBP_CUDA(ctx, cudaMemcpyAsync(ctx->targets.ptr, targets, sizeof(sarbp_target) * nt, cudaMemcpyHostToDevice, s),
                    "upload targets");
@@ -1665,6 +1751,7 @@ sarbp_status sarbp_synthesize_echo(sarbp_ctx *ctx, const sarbp_radar *radar, con
     float2 *d_echo = reinterpret_cast<float2 *>(echo_out);
     const bool dev_out = is_device_ptr(echo_out);
     if (!dev_out) {
+        SARBP_BEGIN(use, kStaging);
         SARBP_CUDA(ctx, ctx->echo.ensure(sizeof(float2) * (size_t)np * ns), "alloc echo");
         d_echo = ctx->echo.as<float2>();
         any_host = true;

@@ -47,3 +47,16 @@ def test_first_call_of_a_context(run, name):
     """Tables and state uploaded for the first call are on the device before its launches read them."""
     rc, out = run("first", name)
     assert rc == 0, out
+
+
+@pytest.mark.parametrize("name", [n for n in CALLS if n != "rc_32768"])
+def test_calls_on_streams_of_their_own(run, name):
+    """A call, each other call and the first again, on three streams, without a wait between them."""
+    rc, out = run("streams", name, "rc_32768")
+    assert rc == 0, out
+
+
+def test_call_behind_a_failed_one(run):
+    """What a failing call had queued is ordered before the next call too."""
+    rc, out = run("failed")
+    assert rc == 0, out
