@@ -318,6 +318,9 @@ sarbp_status ensure_tables(sarbp_ctx *ctx, const sarbp_radar *r, const sarbp_rc_
     const int N = lay.nfft, L = r->upsample;
     std::vector<float2> g, et;
     sarbp::rc_tables_host(*r, lay, g, et);
+    // launches of earlier calls may still read the tables (every call that does uses kRows)
+    if (ctx->shared_used[kRows])
+        SARBP_CUDA(ctx, cudaEventSynchronize(ctx->ev_shared[kRows]), "wait for the tables' last use");
     SARBP_CUDA(ctx, t.filt.ensure(sizeof(float2) * N), "alloc filter");
     SARBP_CUDA(ctx, t.etab.ensure(sizeof(float2) * et.size()), "alloc phase table");
     SARBP_CUDA(ctx, upload(ctx, t.filt.ptr, g.data(), sizeof(float2) * N), "upload filter");
@@ -709,6 +712,8 @@ sarbp_status get_dft(sarbp_ctx *ctx, int n, sarbp::DftPlan &p) {
             if (c.used < slot->used) slot = &c;
         std::vector<float2> etab, chirp, kf, ki;
         sarbp::dft_tables_host(n, etab, chirp, kf, ki);
+        // row transforms on any stream may still read the tables that make room
+        if (slot->n) SARBP_CUDA(ctx, cudaDeviceSynchronize(), "wait for the DFT tables' last use");
         slot->n = 0;
         SARBP_CUDA(ctx, slot->etab.ensure(sizeof(float2) * etab.size()), "alloc DFT tables");
         SARBP_CUDA(ctx, upload(ctx, slot->etab.ptr, etab.data(), sizeof(float2) * etab.size()), "upload DFT tables");

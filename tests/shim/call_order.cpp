@@ -534,10 +534,9 @@ int main(int argc, char **argv) {
     sarbp_ctx *c = context();
     if (what == "first") {  // a call right after sarbp_create
         bad += call(argv[2], c, stream(), false);
-    } else if (what == "streams") {  // argv[2] and every other call (but argv[3]) behind it, each on a stream of its own
-        const std::string name = argv[2], skip = argc > 3 ? argv[3] : "";
+    } else if (what == "streams") {  // argv[2] with every other call behind it, each on a stream of its own
+        const std::string name = argv[2];
         for (auto &kv : kCalls) {
-            if (kv.first == skip) continue;
             cudaDeviceSynchronize();
             g_log.clear();
             const int before = g_conflicts;

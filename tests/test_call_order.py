@@ -49,14 +49,27 @@ def test_first_call_of_a_context(run, name):
     assert rc == 0, out
 
 
-@pytest.mark.parametrize("name", [n for n in CALLS if n != "rc_32768"])
+@pytest.mark.parametrize("name", CALLS)
 def test_calls_on_streams_of_their_own(run, name):
     """A call, each other call and the first again, on three streams, without a wait between them."""
-    rc, out = run("streams", name, "rc_32768")
+    rc, out = run("streams", name)
     assert rc == 0, out
 
 
 def test_call_behind_a_failed_one(run):
     """What a failing call had queued is ordered before the next call too."""
     rc, out = run("failed")
+    assert rc == 0, out
+
+
+@pytest.mark.parametrize("name", ["rc", "rc_fp16", "rc_32768", "rc_host", "image", "image_fp16", "image_host", "dft", "dft2d",
+                                  "wk", "wk_focus"])
+def test_tables_are_not_replaced_under_queued_launches(run, name):
+    """Two sets of parameters in turn, queued without a wait on one stream and on two."""
+    rc, out = run("tables", name)
+    assert rc == 0, out
+
+
+def test_more_dft_lengths_than_kept_tables(run):
+    rc, out = run("lengths")
     assert rc == 0, out

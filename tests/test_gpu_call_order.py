@@ -1,6 +1,6 @@
 """Calls of one context queued back to back without a wait, on streams of their
-own: none may touch the context's scratch while an earlier call still uses it.
-Every result has the bits of the same call alone."""
+own: none may touch the context's scratch, or replace its tables, while an
+earlier call still uses them.  Every result has the bits of the same call alone."""
 import numpy as np
 import pytest
 
@@ -18,7 +18,7 @@ def bits(torch, x):
     return (torch.view_as_real(x) if x.is_complex() else x).view(torch.int16)
 
 
-def check(torch, ctx, calls):
+def check(torch, ctx, calls, one_stream=False):
     """calls: (queue(stream), outputs) pairs; each alone, then all in flight at once, three times."""
     alone = []
     for queue, outs in calls:
@@ -26,7 +26,7 @@ def check(torch, ctx, calls):
         queue(torch.cuda.Stream().cuda_stream)
         torch.cuda.synchronize()
         alone.append([o.clone() for o in outs])
-    streams = [torch.cuda.Stream() for _ in calls]
+    streams = [torch.cuda.Stream() for _ in range(1 if one_stream else len(calls))] * (len(calls) if one_stream else 1)
     for _ in range(3):
         for _, outs in calls:
             for o in outs:
@@ -91,3 +91,33 @@ def test_transposed_transforms(torch):
                 ctx.dft2d(out, stream=st)
             calls.append((dft, [out]))
         check(torch, ctx, calls)
+
+
+@pytest.mark.parametrize("one_stream", [True, False])
+def test_parameters_change_between_queued_calls(torch, one_stream):
+    with sarbp.Context(0) as ctx:
+        calls = []
+        for k in range(4):  # one layout, other chirps: the same tables' memory
+            radar = scenes.Radar(bandwidth=100e6 if k % 2 else 90e6)
+            r = sarbp.radar_struct(radar, 3e-5)
+            echo = noise(torch, k, 1500, 2500)
+            out = torch.zeros(1500, 8 * 2500, dtype=torch.complex64, device="cuda")
+            calls.append((lambda s, r=r, e=echo, o=out: ctx.range_compress(r, e, out=o, stream=s), [out]))
+        check(torch, ctx, calls, one_stream)
+        assert not torch.equal(calls[0][1][0], calls[1][1][0])
+
+
+@pytest.mark.parametrize("one_stream", [True, False])
+def test_more_dft_lengths_than_kept_tables(torch, one_stream):
+    with sarbp.Context(0) as ctx:
+        calls = []
+        for k, n in enumerate((1000, 1024, 1500, 2048, 3000, 999)):
+            x = noise(torch, k, 4000, n)
+            out = torch.zeros_like(x)
+
+            def dft(st, x=x, out=out):
+                with torch.cuda.stream(torch.cuda.ExternalStream(st)):
+                    out.copy_(x)
+                ctx.dft(out, stream=st)
+            calls.append((dft, [out]))
+        check(torch, ctx, calls, one_stream)
