@@ -115,11 +115,8 @@ struct sarbp_ctx {
     std::string err;
     DevBuf echo, spec, rc, scale, apc, image, partial, errword, power, targets, pref;
     DevBuf corr, weight, proj, projout, sharp;  // per-pulse corrections, projection and autofocus scratch
-    DevBuf wk0, wk1, wkrow;                       // omega-K ping-pong buffers, CEOS gain table
+    DevBuf wk0, wk1;                              // omega-K ping-pong buffers
     WkCache wkc;                                  // omega-K tables
-    bool ceos_valid = false;                      // wkrow holds the CEOS gains of ceos_gain
-    float ceos_gain = 0.f;
-    cudaEvent_t ceos_ready = nullptr;             // their upload
     DftCache dft[4];
     uint64_t dft_clock = 0;
     RcTables tables;
@@ -136,7 +133,7 @@ struct sarbp_ctx {
     std::vector<DevBuf *> scratch() {
         std::vector<DevBuf *> v = {&echo,   &spec,  &rc,      &scale,   &apc,     &image,   &partial,
                                    &targets, &pref,  &corr,    &weight,  &proj,    &projout, &sharp,
-                                   &wk0,    &wk1,   &wkrow,   &wkc.row, &wkc.tab};
+                                   &wk0,    &wk1,   &wkc.row, &wkc.tab};
         for (DftCache &d : dft)
             for (DevBuf *b : {&d.etab, &d.chirp, &d.kf, &d.ki}) v.push_back(b);
         return v;
@@ -147,7 +144,6 @@ struct sarbp_ctx {
         for (DevBuf *b : scratch()) b->release();
         for (DftCache &d : dft) d.release();  // also forgets the cached sizes
         wkc.valid = false;
-        ceos_valid = false;
     }
     int64_t launches = 0;
     sarbp::Tuning tune;           // sarbp_debug_set: forced chunk / segments, checked kernels, wait faults
@@ -826,7 +822,6 @@ sarbp_status sarbp_destroy(sarbp_ctx *ctx) {
         if (e) cudaEventDestroy(e);
     if (ctx->ev_ext) cudaEventDestroy(ctx->ev_ext);
     if (ctx->wkc.ready) cudaEventDestroy(ctx->wkc.ready);
-    if (ctx->ceos_ready) cudaEventDestroy(ctx->ceos_ready);
     if (ctx->ev_copy) cudaEventDestroy(ctx->ev_copy);
     for (cudaEvent_t e : ctx->ev_shared)
         if (e) cudaEventDestroy(e);
@@ -1576,25 +1571,14 @@ sarbp_status sarbp_ceos_decode(sarbp_ctx *ctx, const uint8_t *raw, uint64_t raw_
         g.raw_offset = b0 * g.block_bytes;
         any_host = true;
     }
-    // gain per AGC code: float(gain) * float(10^(dB / 20)), the reader's float
-    // arithmetic; uploaded when the layout's gain changes, else reused
-    if (ctx->ceos_valid && ctx->ceos_gain == l->gain) {
-        SARBP_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ceos_ready, 0), "gain table");
-    } else {
-        ctx->ceos_valid = false;
-        float gains[64];
-        for (int code = 0; code < 64; ++code) {
-            const int db = code - 24 * (code > 31);
-            gains[code] = l->gain * (float)std::pow(10.0, db / 20.0);
-        }
-        SARBP_CUDA(ctx, ctx->wkrow.ensure(sizeof gains), "alloc gain table");
-        SARBP_CUDA(ctx, cudaMemcpyAsync(ctx->wkrow.ptr, gains, sizeof gains, cudaMemcpyHostToDevice, s), "upload gains");
-        if (!ctx->ceos_ready)
-            SARBP_CUDA(ctx, cudaEventCreateWithFlags(&ctx->ceos_ready, cudaEventDisableTiming), "gain table");
-        SARBP_CUDA(ctx, cudaEventRecord(ctx->ceos_ready, s), "gain table");
-        ctx->ceos_gain = l->gain;
-        ctx->ceos_valid = true;
-    }
+    // gain per AGC code: float(gain) * float(10^(dB / 20)), the reader's float arithmetic
+    static const sarbp::CeosGains unit = [] {
+        sarbp::CeosGains u;
+        for (int code = 0; code < 64; ++code) u.of_code[code] = (float)std::pow(10.0, (code - 24 * (code > 31)) / 20.0);
+        return u;
+    }();
+    sarbp::CeosGains gains;
+    for (int code = 0; code < 64; ++code) gains.of_code[code] = l->gain * unit.of_code[code];
     float2 *d_echo = reinterpret_cast<float2 *>(echo);
     const size_t out_bytes = sizeof(float2) * (size_t)nlines * ncells;
     const bool dev_echo = is_device_ptr(echo);
@@ -1615,7 +1599,7 @@ sarbp_status sarbp_ceos_decode(sarbp_ctx *ctx, const uint8_t *raw, uint64_t raw_
             any_host = true;
         }
     }
-    SARBP_CUDA(ctx, sarbp::launch_ceos_decode(d_raw, g, ctx->wkrow.as<float>(), d_echo, d_agc, s), "CEOS decode");
+    SARBP_CUDA(ctx, sarbp::launch_ceos_decode(d_raw, g, gains, d_echo, d_agc, s), "CEOS decode");
     ctx->launches += 1;
     if (!dev_echo) SARBP_CUDA(ctx, cudaMemcpyAsync(echo, d_echo, out_bytes, cudaMemcpyDeviceToHost, s), "download echo");
     if (agc_db && d_agc != reinterpret_cast<short *>(agc_db))

@@ -16,7 +16,9 @@
 // Decode (read_CEOS_raw.m:135-141): d = byte & 15, value 2 (d - 16 [d > 7]) + 1.
 // AGC (extract_AGC.m:45-58): code = aux byte agc_byte & 63,
 // dB = code - 24 [code > 31]; gain 1.5 10^(dB / 20) (load_DATA_block.m:58-69),
-// taken from a 64-entry host table so device and host agree bit for bit.
+// taken from a 64-entry host table so device and host agree bit for bit.  The
+// table is a kernel argument (a line's code, and so its entry, is the same for a
+// whole block): each launch has its own, and none waits for an upload.
 #include "sarbp_internal.h"
 
 namespace sarbp {
@@ -29,7 +31,7 @@ __device__ __forceinline__ float ceos_value(unsigned d) {
     return (float)(2 * (v - 16 * (v > 7)) + 1);
 }
 
-__global__ void ceos_decode_kernel(const unsigned char *__restrict__ raw, CeosGeom g, const float *__restrict__ gains,
+__global__ void ceos_decode_kernel(const unsigned char *__restrict__ raw, CeosGeom g, const __grid_constant__ CeosGains gains,
                                    float2 *__restrict__ echo, short *__restrict__ agc_db) {
     const int line = blockIdx.y;                       // 0-based within the request
     const int gl = g.first_line + line;                // line index in the file
@@ -39,7 +41,7 @@ __global__ void ceos_decode_kernel(const unsigned char *__restrict__ raw, CeosGe
     const long long aux_off = base + g.header + g.agc_byte - 1 + (k > r ? g.replica : 0);
     const long long smp_off = base + g.header + g.aux + (k >= r ? g.replica : 0) + 2LL * g.first_cell;
     const unsigned code = raw[aux_off] & 63u;
-    const float gain = g.apply_agc ? gains[code] : 1.f;
+    const float gain = g.apply_agc ? gains.of_code[code] : 1.f;
     if (agc_db && blockIdx.x == 0 && threadIdx.x == 0) agc_db[line] = (short)((int)code - 24 * (code > 31u));
     const unsigned short *s = reinterpret_cast<const unsigned short *>(raw + smp_off);
     float2 *dst = echo + (size_t)line * g.ncells;
@@ -63,7 +65,7 @@ __global__ void ceos_decode_kernel(const unsigned char *__restrict__ raw, CeosGe
 
 }  // namespace
 
-cudaError_t launch_ceos_decode(const unsigned char *raw, const CeosGeom &g, const float *gains, float2 *echo,
+cudaError_t launch_ceos_decode(const unsigned char *raw, const CeosGeom &g, const CeosGains &gains, float2 *echo,
                                short *agc_db, cudaStream_t s) {
     if (g.nlines <= 0 || g.ncells <= 0) return cudaSuccess;
     const int threads = 256;

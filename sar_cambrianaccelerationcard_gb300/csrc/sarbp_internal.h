@@ -372,8 +372,11 @@ struct CeosGeom {
     long long line_bytes, block_bytes;
     long long raw_offset;  // offset of the device buffer's byte 0 from the start of the first block
 };
-// echo [nlines][ncells], agc_db [nlines] (may be null); gains[64] = 1.5 10^(dB(code)/20)
-cudaError_t launch_ceos_decode(const unsigned char *raw, const CeosGeom &g, const float *gains, float2 *echo,
+struct CeosGains {
+    float of_code[64];  // 1.5 10^(dB(code)/20)
+};
+// echo [nlines][ncells], agc_db [nlines] (may be null)
+cudaError_t launch_ceos_decode(const unsigned char *raw, const CeosGeom &g, const CeosGains &gains, float2 *echo,
                                short *agc_db, cudaStream_t s);
 
 // ---------------------------------------------------------------- autofocus (autofocus.cu)

@@ -306,16 +306,12 @@ cudaError_t launch_wk_stolt(const float2 *in, float2 *out, int NA, int NR, const
     op.w(out, 8ull * NA * NR);
     return cudaSuccess;
 }
-static void decode(const unsigned char *raw, const CeosGeom &g, const float *gains, float2 *echo, short *agc, cudaStream_t s) {
+cudaError_t launch_ceos_decode(const unsigned char *raw, const CeosGeom &g, const CeosGains &, float2 *echo, short *agc,
+                               cudaStream_t s) {
     Op op(s, "CEOS decode");
     op.r(raw, (size_t)g.nlines * g.line_bytes);
-    if (on_device(gains)) op.r(gains, 256);
     op.w(echo, 8ull * g.nlines * g.ncells);
     op.w(agc, 2ull * g.nlines);
-}
-cudaError_t launch_ceos_decode(const unsigned char *raw, const CeosGeom &g, const float *gains, float2 *echo, short *agc,
-                               cudaStream_t s) {
-    decode(raw, g, gains, echo, agc, s);
     return cudaSuccess;
 }
 cudaError_t launch_echo_synth(const double *apc, int np, int ns, const sarbp_target *tg, int nt, double, double, double,

@@ -63,7 +63,7 @@ def test_call_behind_a_failed_one(run):
 
 
 @pytest.mark.parametrize("name", ["rc", "rc_fp16", "rc_32768", "rc_host", "image", "image_fp16", "image_host", "dft", "dft2d",
-                                  "wk", "wk_focus"])
+                                  "wk", "wk_focus", "ceos", "ceos_host"])
 def test_tables_are_not_replaced_under_queued_launches(run, name):
     """Two sets of parameters in turn, queued without a wait on one stream and on two."""
     rc, out = run("tables", name)
