@@ -1048,15 +1048,20 @@ cudaError_t launch_split(const BpPlan &p, cudaStream_t s, int tiles, int tiles_y
 }
 
 // A plan asks for the test variants when it carries a fault or a wait limit
-// other than the default (sarbp_debug_set); they exist for 8-pixel columns.
+// other than the default (sarbp_debug_set); they exist for 8-pixel columns, with
+// the staging schemes of production (helper_warps): two helpers for 16-pulse
+// chunks, one for smaller ones, none for FP64 and FP32.  Their phase is the series form.
 bool bp_testing(const BpPlan &p) { return p.fault_chunk >= 0 || p.wait_ns != kDefaultWaitNs; }
 
 template <int MODE, int STORE, bool ADJ>
 cudaError_t launch_testf_mode(const BpPlan &p, cudaStream_t s, int tiles, int tiles_y, int pps, float qq_max) {
-    if constexpr (MODE == SARBP_MODE_SPLIT || MODE == SARBP_MODE_FP16STORE)
+    if constexpr (MODE == SARBP_MODE_SPLIT || MODE == SARBP_MODE_FP16STORE) {
+        if (p.chunk == kChunk)
+            return p.nterms == 3 ? launch_variant<MODE, STORE, 3, false, 8, ADJ, kChunk, true>(p, s, tiles, tiles_y, pps, qq_max)
+                                 : launch_variant<MODE, STORE, 4, false, 8, ADJ, kChunk, true>(p, s, tiles, tiles_y, pps, qq_max);
         return p.nterms == 3 ? launch_variant<MODE, STORE, 3, false, 8, ADJ, 0, true>(p, s, tiles, tiles_y, pps, qq_max)
                              : launch_variant<MODE, STORE, 4, false, 8, ADJ, 0, true>(p, s, tiles, tiles_y, pps, qq_max);
-    else
+    } else
         return launch_variant<MODE, STORE, 4, false, 8, false, 0, true>(p, s, tiles, tiles_y, pps, qq_max);
 }
 
