@@ -664,10 +664,6 @@ __device__ __forceinline__ void fft_io_group(float2 *s, const Etab &E,
 // of the inverse range transform.
 constexpr int kWhiMax = 128, kRampMax = 64;
 constexpr size_t kTabSmem = sizeof(float2) * (kWlo + kWhiMax + kRampMax);
-template <int N>
-__device__ __forceinline__ float2 *ramp_slots(float2 *sm) {
-    return sm + N + kWlo + kWhiMax;
-}
 
 // Fills the W tables (W^m = E^{L m}) straight from the global E table, which the
 // CTAs of an SM share in L1: no barrier here (the caller synchronises before the
@@ -675,20 +671,23 @@ __device__ __forceinline__ float2 *ramp_slots(float2 *sm) {
 // 18 KB per CTA, a barrier before the W tables could be derived and 15% of the
 // shared wavefronts: range compression of 4096 16384-point pulses 2.84 -> 2.74 ms,
 // 8192 points -4%, omega-K image 816 -> 799 us.
-template <int N, int T, int BLOCK = T>
-__device__ __forceinline__ Etab load_etab_at(float2 *tables, const float2 *__restrict__ etab, int L) {
+// fill_w: the W tables by the block's threads from any source e of E^m.
+template <int N, int BLOCK, class Power>
+__device__ __forceinline__ void fill_w(float2 *tables, int L, Power e) {
     static_assert(N / kWlo <= kWhiMax, "W table too small");
-    float2 *wlo = tables;
-    float2 *whi = wlo + kWlo;
-    const Etab E{etab, wlo, whi};
     constexpr int nwlo = N < kWlo ? N : kWlo;
     constexpr int nwhi = N < kWlo ? 1 : N / kWlo;
     for (int i = threadIdx.x; i < nwlo + nwhi; i += BLOCK) {
         if (i < nwlo)
-            wlo[i] = E(L * i);
+            tables[i] = e(L * i);
         else
-            whi[i - nwlo] = E((L * kWlo * (i - nwlo)) & (L * N - 1));
+            tables[kWlo + i - nwlo] = e((L * kWlo * (i - nwlo)) & (L * N - 1));
     }
+}
+template <int N, int T, int BLOCK = T>
+__device__ __forceinline__ Etab load_etab_at(float2 *tables, const float2 *__restrict__ etab, int L) {
+    const Etab E{etab, tables, tables + kWlo};
+    fill_w<N, BLOCK>(tables, L, E);
     return E;
 }
 // Tables right after the N points of a single transform at sm.

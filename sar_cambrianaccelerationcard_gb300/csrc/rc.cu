@@ -113,7 +113,25 @@ __global__ void __launch_bounds__(T, (fft_min_blocks<N, T>())) rc_forward_kernel
 // each, from disjoint banks
 template <int G>
 constexpr int group_pad = G > 1 ? 16 / G : 0;
-template <int N, int M, int T, int G, int STORE>
+// The ramp factors into two levels (per thread, per phase) where every first-stage
+// point of a thread is congruent to its index modulo T: all but the transforms of
+// 64 to 256 points, which read E^{kappa r} point by point.
+template <int N, int M, int T>
+constexpr bool two_level_ramp = (N / 2) % T == 0 && N / T <= kRampMax && FirstIn<M, T>::NB % T == 0;
+// STAGED copies the E table to shared memory, a spare slot per 8 entries.  At 16x
+// upsampling the strides of W^m = E^{16 m} and of the point-by-point ramp put
+// every lane on a line of its own, and gathers from global memory bound the
+// transforms of 128 and 256 points: 8192 pulses, complex64 / FP16 rows, 253 / 226 us
+// from global, 210 / 214 staged (128 points), 348 / 289 and 295 / 249 (256).  64
+// points have too few gathers to pay for the copy (175 / 191 against 182 / 201); at 8x
+// reading from global memory is the faster one (256 points: 140 -> 134 us).
+template <int N>
+constexpr bool staged_at_16x = N == 128 || N == 256;
+constexpr int kStagedTable = 256 + 16;  // entries at 256 points and 16x
+__device__ __forceinline__ int tslot(int i) { return i + (i >> 3); }
+constexpr int kStagedSlots = kStagedTable + kStagedTable / 8;
+
+template <int N, int M, int T, int G, int STORE, bool STAGED>
 __global__ void __launch_bounds__(G *T, (fft_min_blocks<G * M, G * T>()))
     rc_inverse_kernel(int L, int nbins, const float2 *__restrict__ spec, const float2 *__restrict__ etab,
                       const float *__restrict__ bound2, float *__restrict__ scale, void *__restrict__ out) {
@@ -134,14 +152,21 @@ __global__ void __launch_bounds__(G *T, (fft_min_blocks<G * M, G * T>()))
         for (int q = 0; q < F::R; ++q)
             v[b][q] = F::live(b, tid) ? __ldg(&in[F::point(b, q, tid)]) : make_float2(0.f, 0.f);
     float2 *tables = sm + G * CS;
-    const Etab E = load_etab_at<M, T, G * T>(tables, etab, LF);
+    constexpr bool kTwoLevel = two_level_ramp<N, M, T>;
+    static_assert(kTwoLevel ? !STAGED : FOLD == 1 && G == 1 && N <= 256, "point-by-point ramp: small single transforms");
+    float2 *et = tables + kWlo + kWhiMax + kRampMax;
+    auto staged_e = [&](int m) { return cmul(et[tslot(256 + (m >> 8))], et[tslot(m & 255)]); };
+    if (STAGED) {
+        for (int i = threadIdx.x; i < 256 + LN / 256; i += T) et[tslot(i)] = __ldg(&etab[i]);
+        __syncthreads();
+        fill_w<M, T>(tables, L, staged_e);
+    }
+    const Etab E = STAGED ? Etab{etab, tables, tables + kWlo} : load_etab_at<M, T, G * T>(tables, etab, LF);
     // Ramp E^{kappa r}, kappa the signed frequency (MATLAB split floor((N+1)/2)
     // = N/2 for even N).  With k = tid + T i (every first-stage point of a
     // thread is congruent to tid mod T when M / R is a multiple of T) and N/2 a
     // multiple of T it factors into a per-thread E^{tid r} and a per-phase table
     // over i that also carries the E^{-N r} of the negative half.
-    constexpr bool kTwoLevel = (N / 2) % T == 0 && N / T <= kRampMax && F::NB % T == 0;
-    static_assert(kTwoLevel || FOLD == 1, "folded spectra use the two-level ramp");
     float2 *rt = tables + kWlo + kWhiMax + group * kRampMax;
     float2 base = make_float2(1.f, 0.f);
     if (kTwoLevel && r != 0) {
@@ -153,7 +178,7 @@ __global__ void __launch_bounds__(G *T, (fft_min_blocks<G * M, G * T>()))
         }
         base = E((tid * r) & (LN - 1));
     }
-    __syncthreads();
+    if (kTwoLevel) __syncthreads();  // the ramp table; the W tables are read behind the first stage's barrier
     if (r != 0) {
 #pragma unroll
         for (int b = 0; b < F::PER; ++b)
@@ -163,8 +188,8 @@ __global__ void __launch_bounds__(G *T, (fft_min_blocks<G * M, G * T>()))
                 if (kTwoLevel) {
                     v[b][q] = cmul(v[b][q], rt[k / T]);
                 } else {
-                    const int kap = k < N / 2 ? k : k - N;
-                    v[b][q] = cmul(v[b][q], E((kap * r) & (LN - 1)));  // LN is a power of two
+                    const int m = ((k < N / 2 ? k : k - N) * r) & (LN - 1);  // LN is a power of two
+                    v[b][q] = cmul(v[b][q], STAGED ? staged_e(m) : E(m));
                 }
             }
 #pragma unroll
@@ -304,12 +329,13 @@ cudaError_t fwd_n(const RcPlan &p, const float2 *echo, const float2 *filt, const
     return cudaGetLastError();
 }
 
-template <int N, int STORE, int G>
+template <int N, int STORE, int G, bool STAGED = false>
 cudaError_t inv_g(const RcPlan &p, const float2 *spec, const float2 *etab, const float *bound2, float *scale,
                   void *out, cudaStream_t s) {
     constexpr int M = N < kInvPoints ? N : kInvPoints, T = threads_for<M>();
-    const size_t smem = sizeof(float2) * (G * (M + group_pad<G>) + (G - 1) * kRampMax) + kTabSmem;
-    auto k = rc_inverse_kernel<N, M, T, G, STORE>;
+    constexpr int slots = G * (M + group_pad<G>) + (G - 1) * kRampMax + (STAGED ? kStagedSlots : 0);
+    const size_t smem = sizeof(float2) * slots + kTabSmem;
+    auto k = rc_inverse_kernel<N, M, T, G, STORE, STAGED>;
     cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void *>(k));
     if (e != cudaSuccess || t_prepare) return e;
     k<<<p.np * (p.L * (N / M) / G), G * T, smem, s>>>(p.L, p.nbins, spec, etab, bound2, scale, out);
@@ -318,6 +344,9 @@ cudaError_t inv_g(const RcPlan &p, const float2 *spec, const float2 *etab, const
 template <int N, int STORE>
 cudaError_t inv_s(const RcPlan &p, const float2 *spec, const float2 *etab, const float *bound2, float *scale,
                   void *out, cudaStream_t s) {
+    if constexpr (staged_at_16x<N>) {
+        if (p.L == 16) return inv_g<N, STORE, 1, true>(p, spec, etab, bound2, scale, out, s);
+    }
     constexpr int G = phases_for<N, STORE>();
     if (p.L % G == 0) return inv_g<N, STORE, G>(p, spec, etab, bound2, scale, out, s);
     return inv_g<N, STORE, 1>(p, spec, etab, bound2, scale, out, s);

@@ -1,0 +1,39 @@
+"""Range compression on both sides of the rules that choose a launch's layout,
+against the FP64 oracle: short transforms at 16x upsampling, whose phase table goes
+through shared memory at 128 and 256 points.  Tolerances of the size sweep
+(tests/test_gpu_rc_sizes.py): complex64 rows -110 dB, FP16 rows -60 dB."""
+import numpy as np
+import pytest
+
+from sar_cambrianaccelerationcard_gb300 import metrics, sarbp, scenes
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    with sarbp.Context(0) as c:
+        yield c
+
+
+def against_oracle(ctx, orc, tp, ns, L, n_p):
+    s = scenes.config1(np_=n_p, ns=ns, n_img=8)
+    s.radar = scenes.Radar(tp=tp, upsample=L)
+    s.t_rec0 = scenes.centred_record_start(s.radar, ns)
+    rng = np.random.default_rng(ns + L)
+    echo = (rng.standard_normal((n_p, ns)) + 1j * rng.standard_normal((n_p, ns))).astype(np.complex64)
+    ref = orc.range_compress(s, echo.astype(np.complex128))
+    r, _, _ = sarbp.scene_args(s)
+    rc = ctx.range_compress(r, echo)
+    h, scale = ctx.range_compress(r, echo, storage=sarbp.STORE_C32H)
+    rc16 = (h[..., 0].astype(np.float64) + 1j * h[..., 1].astype(np.float64)) * scale[:, None]
+    assert metrics.rel_l2_db(rc, ref) <= -110.0
+    assert metrics.rel_l2_db(rc16, ref) <= -60.0
+
+
+@pytest.mark.parametrize("nfft", [64, 128, 256, 512])
+@pytest.mark.parametrize("L", [8, 16])
+def test_short_transforms(ctx, orc, nfft, L):
+    tp = 0.05e-6  # 6 samples
+    against_oracle(ctx, orc, tp, nfft - 6, L, 5)
+    against_oracle(ctx, orc, tp, nfft // 2 - 3, L, 5)  # the shortest rows of the size
