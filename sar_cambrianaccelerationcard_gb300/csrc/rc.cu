@@ -307,10 +307,26 @@ constexpr int threads_for() {
 // phase's bins lie L bins apart, so a warp's store touches 16 lines of 128 bytes;
 // two phases' neighbouring bins halve that, which pays while the shared-memory and
 // store path bounds the kernel and the larger CTA costs no residency (two
-// 16384-point phases do not fit one SM).  Rows are divided evenly: L % G == 0.
+// 16384-point phases do not fit one SM).
 template <int N, int STORE>
 constexpr int phases_for() {
     return N == 4096 || (N == 8192 && STORE == SARBP_STORE_C64) ? 2 : 1;
+}
+// Whether a launch takes pairs where the length has them (same bits either way).  Rows
+// divide evenly: L % 2 == 0.  While single phases have an SM each, pairs only make
+// each CTA longer (us, single / pairs: 16 pulses of 4096 points at 4x 15.9 / 18.0,
+// FP16 19.0 / 21.1; of 8192 points 22.0 / 23.9).  At 8192 points a pair takes an SM
+// alone, single phases share one three ways, so at 2x and 4x, with less of the store
+// path to save, a second wave of pairs has to be half full (2x, 200 pulses 31.3 / 33.4,
+// 304 pulses 35.4 / 33.4), and at 2x beyond two waves single phases win (4096 pulses
+// 318 / 344; at 4x 691 / 643).
+template <int N>
+bool take_pairs(const RcPlan &p) {
+    const long long pairs = (long long)p.np * p.L / 2, sms = current_sms();
+    if (p.L % 2 || 2 * pairs <= sms) return false;
+    if (N < 8192 || p.L > 4) return true;
+    if (pairs > sms && 2 * pairs <= 3 * sms) return false;
+    return p.L == 4 || pairs <= 2 * sms;
 }
 // With t_prepare set the launchers below configure their kernel and return
 // without launching it (prepare_rc_kernels).
@@ -347,8 +363,14 @@ cudaError_t inv_s(const RcPlan &p, const float2 *spec, const float2 *etab, const
     if constexpr (staged_at_16x<N>) {
         if (p.L == 16) return inv_g<N, STORE, 1, true>(p, spec, etab, bound2, scale, out, s);
     }
-    constexpr int G = phases_for<N, STORE>();
-    if (p.L % G == 0) return inv_g<N, STORE, G>(p, spec, etab, bound2, scale, out, s);
+    if constexpr (phases_for<N, STORE>() == 2) {
+        if (t_prepare) {  // both layouts: a later launch may have any number of pulses
+            const cudaError_t e = inv_g<N, STORE, 2>(p, spec, etab, bound2, scale, out, s);
+            if (e != cudaSuccess) return e;
+        } else if (take_pairs<N>(p)) {
+            return inv_g<N, STORE, 2>(p, spec, etab, bound2, scale, out, s);
+        }
+    }
     return inv_g<N, STORE, 1>(p, spec, etab, bound2, scale, out, s);
 }
 template <int N>
