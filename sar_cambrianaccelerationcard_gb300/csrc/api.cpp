@@ -425,13 +425,22 @@ sarbp_status rc_host_echo_enqueue(sarbp_ctx *ctx, const sarbp_radar *r, const sa
     SARBP_CUDA(ctx, cudaEventRecord(ctx->ev_copy, s), "order echo upload");
     SARBP_CUDA(ctx, cudaStreamWaitEvent(ctx->copy_stream, ctx->ev_copy, 0), "order echo upload");
     cudaEventRecord(ctx->ev[0], s);
-    // 256 pulses first (the exposed copy), then chunks half as large again: a
-    // pulse takes about twice as long to compress as to upload (8192-point
-    // transforms 0.30 against 0.16 us at 200 GB/s), so the next copy still hides,
-    // and few, larger launches fill the chip.  1111 pulses of 4000 samples in
-    // chunks of 256: 1378 us for the whole image call, 1353 growing.
+    // 256 pulses first (the exposed copy), then chunks half as large again, for few,
+    // larger launches fill the chip (1111 pulses of 4000 samples at 8x, the whole
+    // image call: 1378 us in chunks of 256, 1353 growing), up to a bound, for the
+    // compression of the last chunk is exposed too.  load is proportional to a
+    // pulse's compression over its upload (200 GB/s over C2C), equal near 9:
+    //  - up to that, an eighth of the pulses costs nothing against equal chunks, more
+    //    does (14000 samples at 2x, 20000 pulses, ms: equal 11.2, an eighth 11.1,
+    //    unbounded 12.2);
+    //  - then 1024 pulses gain (900 samples at 1x, 3000 pulses, us: equal 223, an eighth
+    //    227, 1024 186; 2000 samples at 4x, 8000 pulses: 738, 738, 747, unbounded 831);
+    //  - from twice that on the copies hide behind any chunk (2000 samples at 8x,
+    //    8000 pulses: equal 1105, 1024 1082, unbounded 1038).
+    const long long load = (1 + r->upsample) * (long long)lay.nfft / ns;
+    const int bound = load >= 18 ? np : std::max(load >= 9 ? 1024 : 256, (np + 7) / 8);
     int chunk = 256;
-    for (int p0 = 0, n = 0; p0 < np; p0 += n, chunk += chunk / 2) {
+    for (int p0 = 0, n = 0; p0 < np; p0 += n, chunk = std::min(chunk + chunk / 2, bound)) {
         n = np - p0 < chunk + chunk / 4 ? np - p0 : chunk;  // no small last chunk
         SARBP_CUDA(ctx, cudaMemcpyAsync(d_echo + (size_t)p0 * ns, echo + (size_t)p0 * ns, row * n, cudaMemcpyHostToDevice,
                                         ctx->copy_stream),

@@ -43,6 +43,7 @@ std::map<char *, size_t> g_device;
 std::vector<Access> g_log;
 int g_ids = 0, g_conflicts = 0;
 bool g_fail_bp = false;
+std::vector<size_t> g_uploads;  // bytes of each host-to-device copy
 
 int id_of(const void *h) { return (int)(intptr_t)h; }  // stream and event handles are small integers
 int begin_op(int stream) {
@@ -148,6 +149,7 @@ cudaError_t cudaMemcpyAsync(void *d, const void *src, size_t n, cudaMemcpyKind, 
     Op op(s, "copy");
     if (on_device(src)) op.r(src, n);
     if (on_device(d)) op.w(d, n);
+    if (on_device(d) && !on_device(src)) g_uploads.push_back(n);
     return cudaSuccess;
 }
 cudaError_t cudaMemcpy(void *d, const void *src, size_t n, cudaMemcpyKind k) {
@@ -550,6 +552,13 @@ int main(int argc, char **argv) {
         cudaStream_t s[2] = {stream(), stream()};
         const int n[] = {64, 100, 128, 200, 256, 300, 64, 100};
         for (int k = 0; k < 8; ++k) bad += sarbp_dft(c, device<sarbp_complex64>(10 * n[k]), 10, n[k], 0, s[k & 1]) != SARBP_OK;
+    } else if (what == "uploads") {  // pulses of each chunk of a host echo of argv[2] pulses, argv[3] samples, upsampled by argv[4]
+        const int np = std::atoi(argv[2]), ns = std::atoi(argv[3]);
+        g_uploads.clear();
+        bad += range_compress(c, stream(), false, SARBP_STORE_C32H, true, np, ns, std::atoi(argv[4])) != SARBP_OK;
+        for (size_t n : g_uploads)
+            if (n % (8ull * ns) == 0) std::printf("%zu ", n / (8ull * ns));
+        std::printf("\n");
     } else if (what == "failed") {  // a back-projection that fails behind its first launch
         g_fail_bp = true;
         bad += call("image", c, stream(), false, SARBP_ERR_CUDA);

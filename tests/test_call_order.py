@@ -73,3 +73,22 @@ def test_tables_are_not_replaced_under_queued_launches(run, name):
 def test_more_dft_lengths_than_kept_tables(run):
     rc, out = run("lengths")
     assert rc == 0, out
+
+
+@pytest.mark.parametrize("n_p,ns,L", [(20, 900, 8), (300, 2000, 8), (1111, 4000, 8), (3000, 14000, 2), (3001, 900, 1),
+                                      (8000, 2000, 4), (8000, 6000, 8), (5000, 14000, 1)])
+def test_upload_chunks(run, n_p, ns, L):
+    """A host echo goes up in chunks of 256 pulses and then half as many again, up to
+    an eighth of the pulses, or 1024 where compression takes as long as the copy, or
+    without a bound where it takes twice that; the last chunk, whose compression nothing
+    hides, is no larger than a quarter above the bound."""
+    rc, out = run("uploads", str(n_p), str(ns), str(L))
+    assert rc == 0, out
+    chunks = [int(x) for x in out.splitlines()[0].split()]
+    nfft = 1 << (ns + 1200 - 2).bit_length()
+    load = (1 + L) * nfft // ns
+    bound = n_p if load >= 18 else max(1024 if load >= 9 else 256, -(-n_p // 8))
+    assert sum(chunks) == n_p and chunks[0] == min(n_p, 256 if n_p >= 320 else n_p)
+    assert max(chunks) <= bound + bound // 4
+    for a, b in zip(chunks, chunks[1:-1]):
+        assert a <= b <= a + a // 2
