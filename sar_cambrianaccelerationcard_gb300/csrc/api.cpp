@@ -233,19 +233,20 @@ struct Range {
 // orders it against the context's other calls.
 class ScratchUse {
   public:
-    ScratchUse(sarbp_ctx *ctx, cudaStream_t s) : ctx_(ctx), s_(s) {
-        cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(s, &c) != cudaSuccess) cudaGetLastError();
-        capturing_ = c != cudaStreamCaptureStatusNone;
-    }
+    ScratchUse(sarbp_ctx *ctx, cudaStream_t s) : ctx_(ctx), s_(s) {}
     ScratchUse(const ScratchUse &) = delete;
     ScratchUse &operator=(const ScratchUse &) = delete;
     sarbp_status begin(Shared group) {
-        if (capturing_ || begun_[group]) return SARBP_OK;
+        if (begun_[group] || capturing()) return SARBP_OK;
         if (ctx_->shared_used[group])
             SARBP_CUDA(ctx_, cudaStreamWaitEvent(s_, ctx_->ev_shared[group], 0), "order shared scratch");
         begun_[group] = true;
         return SARBP_OK;
+    }
+    // The stream is idle: this call's accesses, and those it waited for, are over.
+    void finished() {
+        for (int k = 0; k < kSharedGroups; ++k)
+            if (begun_[k]) begun_[k] = ctx_->shared_used[k] = false;
     }
     ~ScratchUse() {
         for (int k = 0; k < kSharedGroups; ++k) {
@@ -256,9 +257,17 @@ class ScratchUse {
     }
 
   private:
+    bool capturing() {
+        if (capture_ < 0) {
+            cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+            if (cudaStreamIsCapturing(s_, &c) != cudaSuccess) cudaGetLastError();
+            capture_ = c != cudaStreamCaptureStatusNone;
+        }
+        return capture_ != 0;
+    }
     sarbp_ctx *ctx_;
     cudaStream_t s_;
-    bool capturing_ = false;
+    int capture_ = -1;  // not asked yet
     bool begun_[kSharedGroups] = {};
 };
 #define SARBP_BEGIN(use, group)                               \
@@ -355,9 +364,10 @@ sarbp_status check_errword(sarbp_ctx *ctx) {
 }
 
 // finish a call: synchronise when host memory is involved, read timings and checks
-sarbp_status finish(sarbp_ctx *ctx, cudaStream_t s, bool sync) {
+sarbp_status finish(sarbp_ctx *ctx, cudaStream_t s, bool sync, ScratchUse &use) {
     if (!sync) return SARBP_OK;
     SARBP_CUDA(ctx, cudaStreamSynchronize(s), "stream synchronize");
+    use.finished();
     if (ctx->timed_rc) cudaEventElapsedTime(&ctx->rc_ms, ctx->ev[0], ctx->ev[1]);
     if (ctx->timed_bp) cudaEventElapsedTime(&ctx->bp_ms, ctx->ev[2], ctx->ev[3]);
     return check_errword(ctx);
@@ -916,7 +926,7 @@ sarbp_status sarbp_range_compress(sarbp_ctx *ctx, const sarbp_radar *radar, cons
     if (storage == SARBP_STORE_C32H && !dev_sc)
         SARBP_CUDA(ctx, cudaMemcpyAsync(rc_scale_out, d_scale, sizeof(float) * np, cudaMemcpyDeviceToHost, s),
                    "download scale");
-    return finish(ctx, s, !dev_in || !dev_out || !dev_sc);
+    return finish(ctx, s, !dev_in || !dev_out || !dev_sc, use);
 }
 
 sarbp_status sarbp_backproject_ex(sarbp_ctx *ctx, const sarbp_radar *radar, const sarbp_rc_view *rc,
@@ -951,7 +961,7 @@ sarbp_status sarbp_backproject_ex(sarbp_ctx *ctx, const sarbp_radar *radar, cons
     if (st != SARBP_OK) return st;
     if (!dev_img)
         SARBP_CUDA(ctx, cudaMemcpyAsync(image, d_img, sizeof(float2) * npix, cudaMemcpyDeviceToHost, s), "download image");
-    return finish(ctx, s, any_host);
+    return finish(ctx, s, any_host, use);
 }
 
 sarbp_status sarbp_bp_plan(sarbp_ctx *ctx, const sarbp_radar *radar, const sarbp_rc_view *rc, const double *apc,
@@ -996,6 +1006,7 @@ sarbp_status sarbp_bp_plan(sarbp_ctx *ctx, const sarbp_radar *radar, const sarbp
         }
         st = extremes_device(ctx, apc_dev, np, grid, ctx->stream, ex);
         if (st != SARBP_OK) return st;
+        use.finished();  // the reduction's result is here, so it and the upload before it are over
     }
     sarbp::BpPlan p;
     std::string why;
@@ -1070,7 +1081,7 @@ sarbp_status sarbp_project_weighted(sarbp_ctx *ctx, const sarbp_radar *radar, co
     }
     if (!dev_out)
         SARBP_CUDA(ctx, cudaMemcpyAsync(out, d_out, sizeof(double2) * np, cudaMemcpyDeviceToHost, s), "download projection");
-    return finish(ctx, s, any_host);
+    return finish(ctx, s, any_host, use);
 }
 
 sarbp_status sarbp_autofocus(sarbp_ctx *ctx, const sarbp_radar *radar, const sarbp_rc_view *rc, const double *apc,
@@ -1095,7 +1106,7 @@ sarbp_status sarbp_autofocus(sarbp_ctx *ctx, const sarbp_radar *radar, const sar
     SARBP_BEGIN(use, kStaging);
     const int np = rc->np;
     const size_t npix = (size_t)grid->nx * grid->ny;
-    if (np == 0 || npix == 0) return finish(ctx, s, true);
+    if (np == 0 || npix == 0) return finish(ctx, s, true, use);
     std::vector<double> ph(dphase, dphase + np);
     for (double v : ph)
         if (!std::isfinite(v)) return fail(ctx, SARBP_ERR_INVALID_ARGUMENT, "dphase must be finite");
@@ -1151,7 +1162,7 @@ sarbp_status sarbp_autofocus(sarbp_ctx *ctx, const sarbp_radar *radar, const sar
     std::copy(ph.begin(), ph.end(), dphase);
     if (image && !dev_img)
         SARBP_CUDA(ctx, cudaMemcpyAsync(image, d_img, sizeof(float2) * npix, cudaMemcpyDeviceToHost, s), "download image");
-    return finish(ctx, s, true);
+    return finish(ctx, s, true, use);
 }
 
 sarbp_status sarbp_wk_padded_size(int32_t na, int32_t nr, int32_t *na_pad, int32_t *nr_pad) {
@@ -1191,7 +1202,7 @@ sarbp_status sarbp_dft(sarbp_ctx *ctx, sarbp_complex64 *data, int32_t rows, int3
                "DFT launch");
     ctx->launches += 1;
     if (!dev) SARBP_CUDA(ctx, cudaMemcpyAsync(data, d, bytes, cudaMemcpyDeviceToHost, s), "download DFT rows");
-    return finish(ctx, s, !dev);
+    return finish(ctx, s, !dev, use);
 }
 
 sarbp_status sarbp_dft2d(sarbp_ctx *ctx, sarbp_complex64 *data, int32_t na, int32_t nr, int32_t inverse,
@@ -1241,7 +1252,7 @@ sarbp_status sarbp_dft2d(sarbp_ctx *ctx, sarbp_complex64 *data, int32_t na, int3
         }
     }
     if (!dev) SARBP_CUDA(ctx, cudaMemcpyAsync(data, d, bytes, cudaMemcpyDeviceToHost, s), "download DFT array");
-    return finish(ctx, s, !dev);
+    return finish(ctx, s, !dev, use);
 }
 
 // Omega-K parameter checks shared by the pipeline and its stage entry points.
@@ -1442,7 +1453,7 @@ sarbp_status sarbp_wk_image(sarbp_ctx *ctx, const sarbp_wk_params *w, const sarb
     ctx->launches += cols ? 4 : 8;  // and the Stolt launch counted by wk_focus_launch
     if (!dev_img)
         SARBP_CUDA(ctx, cudaMemcpyAsync(image, out, sizeof(float2) * npix, cudaMemcpyDeviceToHost, s), "download image");
-    return finish(ctx, s, any_host);
+    return finish(ctx, s, any_host, use);
 }
 
 sarbp_status sarbp_wk_preprocess(sarbp_ctx *ctx, const sarbp_wk_params *w, const sarbp_complex64 *echo, int32_t na,
@@ -1484,7 +1495,7 @@ sarbp_status sarbp_wk_preprocess(sarbp_ctx *ctx, const sarbp_wk_params *w, const
     SARBP_CUDA(ctx, sarbp::launch_wk_pad(d_echo, na, nr, tb.rowphase, pa, pr, NA, NR, d_out, s), "padding");
     ctx->launches += 1;
     if (!dev_out) SARBP_CUDA(ctx, cudaMemcpyAsync(out, d_out, bytes, cudaMemcpyDeviceToHost, s), "download");
-    return finish(ctx, s, true);  // the host tables are staged through pageable memory
+    return finish(ctx, s, true, use);  // the host tables are staged through pageable memory
 }
 
 sarbp_status sarbp_wk_focus(sarbp_ctx *ctx, const sarbp_wk_params *w, const sarbp_complex64 *spectrum, int32_t na_pad,
@@ -1522,7 +1533,7 @@ sarbp_status sarbp_wk_focus(sarbp_ctx *ctx, const sarbp_wk_params *w, const sarb
     st = wk_focus_launch(ctx, w, tb, d_in, d_out, na_pad, nr_pad, s);
     if (st != SARBP_OK) return st;
     if (!dev_out) SARBP_CUDA(ctx, cudaMemcpyAsync(out, d_out, bytes, cudaMemcpyDeviceToHost, s), "download");
-    return finish(ctx, s, true);
+    return finish(ctx, s, true, use);
 }
 
 sarbp_status sarbp_ceos_decode(sarbp_ctx *ctx, const uint8_t *raw, uint64_t raw_bytes,
@@ -1614,7 +1625,7 @@ sarbp_status sarbp_ceos_decode(sarbp_ctx *ctx, const uint8_t *raw, uint64_t raw_
     if (agc_db && d_agc != reinterpret_cast<short *>(agc_db))
         SARBP_CUDA(ctx, cudaMemcpyAsync(agc_db, d_agc, sizeof(short) * nlines, cudaMemcpyDeviceToHost, s),
                    "download agc");
-    return finish(ctx, s, any_host);
+    return finish(ctx, s, any_host, use);
 }
 
 sarbp_status sarbp_image(sarbp_ctx *ctx, const sarbp_radar *radar, const sarbp_complex64 *echo, int32_t np,
@@ -1710,7 +1721,7 @@ sarbp_status sarbp_image(sarbp_ctx *ctx, const sarbp_radar *radar, const sarbp_c
             return cuda_fail(ctx, e, "download image");
         }
     }
-    return finish(ctx, s, any_host);
+    return finish(ctx, s, any_host, use);
 }
 
 sarbp_status sarbp_synthesize_echo(sarbp_ctx *ctx, const sarbp_radar *radar, const double *apc, int32_t np,
@@ -1769,7 +1780,7 @@ sarbp_status sarbp_synthesize_echo(sarbp_ctx *ctx, const sarbp_radar *radar, con
         SARBP_CUDA(ctx, cudaMemcpyAsync(echo_out, d_echo, sizeof(float2) * (size_t)np * ns, cudaMemcpyDeviceToHost, s),
                    "download echo");
     ctx->timed_rc = ctx->timed_bp = false;
-    return finish(ctx, s, any_host);
+    return finish(ctx, s, any_host, use);
 }
 
 // ------------------------------------------------------- reference shims --
