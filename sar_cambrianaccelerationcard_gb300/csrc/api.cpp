@@ -373,6 +373,15 @@ sarbp_status finish(sarbp_ctx *ctx, cudaStream_t s, bool sync, ScratchUse &use) 
     return check_errword(ctx);
 }
 
+// Pulses per launch of a range compression of np pulses: their spectra [batch][nfft]
+// and the split path's per-half bounds [2 batch] fit the scratch, which grows here.
+sarbp_status ensure_spectra(sarbp_ctx *ctx, const sarbp_rc_layout &lay, int np, int *batch) {
+    const size_t row = sizeof(float2) * (size_t)lay.nfft;
+    *batch = (int)std::max<size_t>(1, std::min<size_t>((size_t)np, kSpecScratchBudget / row));
+    SARBP_CUDA(ctx, ctx->spec.ensure((row + sizeof(float) * 2) * (size_t)*batch), "alloc spectrum scratch");
+    return SARBP_OK;
+}
+
 // Range compression of a device-resident echo into a device rc buffer.
 sarbp_status rc_device(sarbp_ctx *ctx, const sarbp_radar *r, const sarbp_rc_layout &lay, const float2 *echo,
                        int np, int ns, int storage, void *rc_out, float *scale_out, cudaStream_t s, ScratchUse &use,
@@ -384,11 +393,9 @@ sarbp_status rc_device(sarbp_ctx *ctx, const sarbp_radar *r, const sarbp_rc_layo
     SARBP_BEGIN(use, kRows);
     sarbp_status st = ensure_tables(ctx, r, lay);
     if (st != SARBP_OK) return st;
-    const size_t row = sizeof(float2) * (size_t)lay.nfft;
-    const int batch = (int)std::max<size_t>(1, std::min<size_t>((size_t)np, kSpecScratchBudget / row));
-    // spectra [batch][nfft], then the split path's per-half bounds [2 batch]
-    SARBP_CUDA(ctx, ctx->spec.ensure(row * (size_t)batch + sizeof(float) * 2 * (size_t)batch), "alloc spectrum scratch");
-    float *bound2 = reinterpret_cast<float *>(static_cast<char *>(ctx->spec.ptr) + row * (size_t)batch);
+    int batch;
+    if ((st = ensure_spectra(ctx, lay, np, &batch)) != SARBP_OK) return st;
+    float *bound2 = reinterpret_cast<float *>(ctx->spec.as<float2>() + (size_t)lay.nfft * batch);
     float *scale = scale_out;
     if (storage == SARBP_STORE_C32H && !scale) return fail(ctx, SARBP_ERR_INVALID_ARGUMENT, "fp16 storage needs a scale array");
     const size_t esize = storage == SARBP_STORE_C64 ? 8 : 4;
@@ -449,9 +456,17 @@ sarbp_status rc_host_echo_enqueue(sarbp_ctx *ctx, const sarbp_radar *r, const sa
     //    8000 pulses: equal 1105, 1024 1082, unbounded 1038).
     const long long load = (1 + r->upsample) * (long long)lay.nfft / ns;
     const int bound = load >= 18 ? np : std::max(load >= 9 ? 1024 : 256, (np + 7) / 8);
-    int chunk = 256;
-    for (int p0 = 0, n = 0; p0 < np; p0 += n, chunk = std::min(chunk + chunk / 2, bound)) {
-        n = np - p0 < chunk + chunk / 4 ? np - p0 : chunk;  // no small last chunk
+    // the spectra of the largest chunk now: growing them in the loop would wait for
+    // the copies and launches in flight, and could fail with part of the work queued
+    int chunk = 256, largest = 0, batch;
+    auto grow = [&] { chunk = std::min(chunk + chunk / 2, bound); };
+    auto size_of = [&](int p0) { return np - p0 < chunk + chunk / 4 ? np - p0 : chunk; };  // no small last chunk
+    for (int p0 = 0; p0 < np; p0 += size_of(p0), grow()) largest = std::max(largest, size_of(p0));
+    const sarbp_status st0 = ensure_spectra(ctx, lay, largest, &batch);
+    if (st0 != SARBP_OK) return st0;
+    chunk = 256;
+    for (int p0 = 0, n = 0; p0 < np; p0 += n, grow()) {
+        n = size_of(p0);
         SARBP_CUDA(ctx, cudaMemcpyAsync(d_echo + (size_t)p0 * ns, echo + (size_t)p0 * ns, row * n, cudaMemcpyHostToDevice,
                                         ctx->copy_stream),
                    "upload echo");

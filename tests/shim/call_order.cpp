@@ -44,6 +44,7 @@ std::vector<Access> g_log;
 int g_ids = 0, g_conflicts = 0;
 bool g_fail_bp = false;
 std::vector<size_t> g_uploads;  // bytes of each host-to-device copy
+int g_frees = 0;
 
 int id_of(const void *h) { return (int)(intptr_t)h; }  // stream and event handles are small integers
 int begin_op(int stream) {
@@ -127,6 +128,7 @@ cudaError_t cudaMalloc(void **p, size_t n) {
     return cudaSuccess;
 }
 cudaError_t cudaFree(void *p) {
+    ++g_frees;
     cudaDeviceSynchronize();
     auto it = g_device.find((char *)p);
     if (it == g_device.end()) return cudaErrorInvalidValue;
@@ -555,10 +557,11 @@ int main(int argc, char **argv) {
     } else if (what == "uploads") {  // pulses of each chunk of a host echo of argv[2] pulses, argv[3] samples, upsampled by argv[4]
         const int np = std::atoi(argv[2]), ns = std::atoi(argv[3]);
         g_uploads.clear();
+        g_frees = 0;
         bad += range_compress(c, stream(), false, SARBP_STORE_C32H, true, np, ns, std::atoi(argv[4])) != SARBP_OK;
         for (size_t n : g_uploads)
             if (n % (8ull * ns) == 0) std::printf("%zu ", n / (8ull * ns));
-        std::printf("\n");
+        std::printf("\n%d buffers freed\n", g_frees);
     } else if (what == "failed") {  // a back-projection that fails behind its first launch
         g_fail_bp = true;
         bad += call("image", c, stream(), false, SARBP_ERR_CUDA);

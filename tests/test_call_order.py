@@ -92,3 +92,11 @@ def test_upload_chunks(run, n_p, ns, L):
     assert max(chunks) <= bound + bound // 4
     for a, b in zip(chunks, chunks[1:-1]):
         assert a <= b <= a + a // 2
+
+
+@pytest.mark.parametrize("n_p,ns,L", [(3000, 900, 8), (8000, 2000, 8), (3000, 14000, 2)])
+def test_first_host_echo_frees_nothing(run, n_p, ns, L):
+    """A context's first host call sizes its scratch once: growing it between chunks would
+    free, and so wait for the copies and launches in flight."""
+    rc, out = run("uploads", str(n_p), str(ns), str(L))
+    assert rc == 0 and out.splitlines()[1] == "0 buffers freed", out
