@@ -288,13 +288,20 @@ int bp_choose_segments(int tiles, int npl, long long npix, int sms, int force) {
 // Small images: where the rule above splits the pulses but its segments leave SMs
 // without a CTA, more of them, down to one chunk of pulses each, until every SM
 // has one (256 pulses onto 128^2 pixels: 8 tiles x 4 segments 22 us, x 16
-// 10.8 us).  Their partial images are small: fewer tiles than SMs.  Apertures
-// the rule keeps in one segment (under 128 pulses) stay there: their sums are
-// one launch in pulse order, without a reduction.
+// 10.8 us).  Where the pulses are no whole number of chunks the last segment holds
+// fewer, if a quarter of the SMs was idle and none gets a second CTA (250 pulses
+// onto 128^2, whole call: 8 segments 48.7 us, 16 43.4; else the extra partial images
+// cost as much as they save: 500 pulses, 16 segments 50.1 us, 32 51.0).  Their partial
+// images are small: fewer tiles than SMs.  Apertures the rule keeps in one segment
+// (under 128 pulses) stay there: their sums are one launch in pulse order, without
+// a reduction.
 int bp_fill_segments(int tiles, int npl, int sms, int segments) {
     const int kc = bp_max_chunk();
     if (segments < 2) return segments;
-    for (int s = segments + 1; s <= 64 && (long long)tiles * segments < sms && npl / s >= kc; ++s) {
+    for (int s = segments + 1; s <= 64 && (long long)tiles * segments < sms; ++s) {
+        if (npl / s < kc &&
+            ((s - 1) * kc >= npl || 4LL * tiles * segments >= 3LL * sms || (long long)tiles * s > sms))
+            break;
         const int pps = ((npl + s - 1) / s + kc - 1) / kc * kc;  // as the launch rounds it
         if ((long long)(s - 1) * pps < npl) segments = s;        // no empty segment
     }
