@@ -35,7 +35,7 @@ def _flags(extra=()):
 def _compile(src: str, extra=(), build_dir: str = BUILD) -> str:
     obj = os.path.join(build_dir, os.path.splitext(src)[0] + ".o")
     path = os.path.join(CSRC, src)
-    deps = [path] + [os.path.join(CSRC, h) for h in os.listdir(CSRC) if h.endswith(".h")] + \
+    deps = [path] + [os.path.join(CSRC, h) for h in os.listdir(CSRC) if h.endswith((".h", ".cuh"))] + \
         [os.path.join(ROOT, "include", "sarbp.h")]
     if os.path.exists(obj) and all(os.path.getmtime(obj) >= os.path.getmtime(d) for d in deps):
         return obj
