@@ -121,3 +121,28 @@ def test_more_dft_lengths_than_kept_tables(torch, one_stream):
                 ctx.dft(out, stream=st)
             calls.append((dft, [out]))
         check(torch, ctx, calls, one_stream)
+
+
+def test_captured_range_compression_replays(torch):
+    """A device-buffer call is captured into a graph after a first one (which uploads the
+    tables and sizes the scratch) and replays on new data."""
+    with sarbp.Context(0) as ctx:
+        r = sarbp.radar_struct(scenes.Radar(upsample=4), 3e-5)
+        a, b = noise(torch, 0, 300, 2500), noise(torch, 1, 300, 2500)
+        echo, out = a.clone(), torch.zeros(300, 4 * 2500, dtype=torch.complex64, device="cuda")
+        torch.cuda.synchronize()
+        ctx.range_compress(r, b, out=out)
+        ctx.synchronize()
+        ref = out.clone()
+        graph = torch.cuda.CUDAGraph()
+        stream = torch.cuda.Stream()
+        with torch.cuda.graph(graph, stream=stream):
+            ctx.range_compress(r, echo, out=out, stream=stream.cuda_stream)
+        echo.copy_(b)
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(torch.view_as_real(out), torch.view_as_real(ref))
+        ctx.range_compress(r, a, out=out)  # the context goes on as before
+        ctx.synchronize()
+        assert not torch.equal(torch.view_as_real(out), torch.view_as_real(ref))
