@@ -39,10 +39,10 @@ FP32_OPS_PER_UPDATE = 19
 MUFU_OPS_PER_UPDATE = 3
 # DRAM bytes (read + write) and L2 bytes (lts__t_bytes.sum) per call, measured by
 # ncu on GB300 for the default workload (4096 pulses x 8192 samples -> 4096^2,
-# complex64 rows): profiles/traffic_bp_rc_config2.md (captured 2026-12-05, one-pass
-# full-size captures of bp_kernel<2,0,3,0,8,0,16,0,0>, rc_forward_kernel<16384,512,0>
-# and rc_inverse_kernel<16384,16384,512,1,0>).  Back-projection: one launch; range
-# compression: two batches of forward + inverse.
+# complex64 rows), one-pass full-size captures of bp_kernel<2,0,3,0,8,0,16,0,0>,
+# rc_forward_kernel<16384,512,0> and rc_inverse_kernel<16384,16384,512,1,0,0> of
+# 2026-12-05.  Back-projection: one launch; range compression: two batches of
+# forward + inverse.
 MEASURED_TRAFFIC = {
     ("full", "split"): {"bp": 234051584 + 115363840,
                         "rc": (134485248 + 209197312 + 268737280 + 1013266432) +
@@ -51,7 +51,7 @@ MEASURED_TRAFFIC = {
 L2_TRAFFIC = {
     ("full", "split"): {"bp": 26029347104, "rc": 815003840 + 8460378976 + 806713632 + 8445957600},
 }
-# ncu's L2 peak for these launches: lts__t_bytes.sum / duration / pct_of_peak (same file)
+# ncu's L2 peak for these launches: lts__t_bytes.sum / duration / pct_of_peak (same captures)
 L2_PEAK_GBS = 26029347104 / 42.431264e-3 / 0.0168 / 1e9
 
 
@@ -463,7 +463,7 @@ def run_ours(args):
         # L2 bytes of the profiled launch over this run's launch time, against ncu's L2 peak
         bw = l2["bp"] / (bp_ms_each * 1e-3) / 1e9
         roofline["l2"] = {"achieved": bw, "peak": L2_PEAK_GBS, "unit": "GB/s", "frac": bw / L2_PEAK_GBS,
-                          "traffic": l2["bp"], "source": "profiles/traffic_bp_rc_config2.md"}
+                          "traffic": l2["bp"], "source": "ncu, one-pass full-size capture"}
     if bp_ms_each and hbm:
         # the same launch against HBM (of measured): algorithmic bytes / launch time
         bw = bp_alg_bytes / (bp_ms_each * 1e-3) / 1e9
@@ -473,11 +473,11 @@ def run_ours(args):
     roofline_rc = {"bound": "hbm", "achieved": rc_bytes / (rc_ms * 1e-3) / 1e9 if rc_ms else None, "peak": hbm,
                    "unit": "GB/s", "frac": (rc_bytes / (rc_ms * 1e-3) / 1e9 / hbm) if (rc_ms and hbm) else None,
                    "traffic": MEASURED_TRAFFIC.get((args.size, args.mode), {}).get("rc"),
-                   "kernel": "rc_forward_kernel<16384,512,false> + rc_inverse_kernel<16384,16384,512,1,0>", "ms": rc_ms}
+                   "kernel": "rc_forward_kernel<16384,512,false> + rc_inverse_kernel<16384,16384,512,1,0,false>", "ms": rc_ms}
     if rc_ms and l2.get("rc"):
         bw = l2["rc"] / (rc_ms * 1e-3) / 1e9
         roofline_rc["l2"] = {"achieved": bw, "peak": L2_PEAK_GBS, "unit": "GB/s", "frac": bw / L2_PEAK_GBS,
-                             "traffic": l2["rc"], "source": "profiles/traffic_bp_rc_config2.md"}
+                             "traffic": l2["rc"], "source": "ncu, one-pass full-size capture"}
     # the transforms themselves: 1 forward + L inverse nfft-point FFTs per pulse at
     # 5 N log2 N flops each, against the live FP32 FMA rate (2 flops per lane)
     fft_flops = scene.np_ * (1 + scene.radar.upsample) * 5.0 * lay.nfft * math.log2(lay.nfft)

@@ -34,10 +34,14 @@
 //      1024^2 at 1.0 m, none / one / two helpers: 1.32 / 1.27 / 1.40 ms; 1.4 m
 //      rotated by 45 degrees 3.06 / 2.65 / 3.84 (3.80 with every warp preparing
 //      parameters); its projection 3.66 / 3.17; 2.2 m onto 512^2 1.50 / 1.27 /
-//      2.08 (1.84); 1200 x 1000 at 0.75 m, rotated 1.61 / 1.56.
+//      2.08 (1.84); 1200 x 1000 at 0.75 m, rotated 1.61 / 1.56.  The helper holds
+//      these to 96 registers as well, and the linear-term ones spill for it: 8 bytes
+//      a thread in back-projection, 4 in the three-term projection.  The times above
+//      include that; what the pixel warps no longer do is worth more.
 //    - The linear-term back-projection with 16-pulse chunks needs more than 96
-//      registers (0.37 m: 0.91 ms without a helper, 0.96 with one), and so do the
-//      FP64 and FP32 comparators; the checked kernels follow.  There the pixel
+//      registers too, but its narrow windows leave a helper little to take over
+//      (0.37 m: 0.91 ms without a helper, 0.96 with one).  The FP64 and FP32
+//      comparators have no helper, and the checked kernels follow.  There the pixel
 //      warps stage, each chunk's parameters by the next warp in turn.
 //  * SPLIT arithmetic per pixel and pulse: with q the pixel offset from the tile
 //    centre, n = 2 q.w + |q|^2 (w = tile centre - APC) and the differential
@@ -45,8 +49,8 @@
 //    of sqrt(1+e); the planner bounds the truncation error) -- all on the FMA
 //    pipe; the phase fma(dR, k_hi, phi_T) + dR k_lo (compensated product); the
 //    only MUFU work is one sin/cos pair.
-//  * What bounds the pixel loop is the register file: a scheduler reads two
-//    32-lane registers per clock, so an FMA of three distinct registers takes
+//  * What bounds the pixel loop is the register file's read ports (57.6% of the issue
+//    slots are used): a scheduler reads two 32-lane registers per clock, so an FMA of three distinct registers takes
 //    1.3-1.5 clk and a packed FP32x2 FMA of three register pairs 3.1, not 2
 //    (microbenchmark; 2.6 with one operand a scalar read as both halves, 2.0
 //    with two).  So per-pulse constants enter the packed operations as scalars
@@ -122,10 +126,10 @@ struct __align__(16) Prm {
     int ws;        // first bin of the window
     int lo, hi;    // copied part of the window [lo, hi) relative to ws
     float scale;   // FP16 storage scale
-    int need;      // (M, d) pairs [0, need) any pixel of the tile reads (the rest are not converted)
-    int unused[4];
+    int need;      // bins [0, need) hold every bin a pixel of the tile reads: (M, d) pairs [0, need - 1)
+    int unused[4]; // keeps the record at the 128 bytes that the planner's bounds count
 };
-// the planner's shared-memory bounds (which windows it accepts) count 128 bytes
+// which windows the planner accepts depends on it through bp_smem_bytes
 static_assert(sizeof(Prm) == 128, "Prm size");
 
 __device__ __forceinline__ float4 lds128(unsigned addr) {
@@ -309,8 +313,8 @@ __device__ __forceinline__ void produce(const BpPlan &P, const Smem &S, int stag
             const int need_end = (int)ceilf(fminf(fmaxf(bT.h + half, -1.0e9f), 1.0e9f)) + 2;
             sane = isfinite(r) && r > 0.f && isfinite(half) && isfinite(phT) && need_end - ws <= win;
             // the tile's bins lie in [bT - half, bT + half]: pair indices up to
-            // need_end - ws - 2, so pairs [0, need) cover every read (the checked
-            // build flags any read past need - 2)
+            // need_end - ws - 2, so pairs [0, need - 1) cover every read (the
+            // checked build flags any read past need - 2)
             if (sane) need = need_end - ws;
             const float i2 = iR * iR;
             if (sane) {

@@ -104,13 +104,8 @@ __global__ void __launch_bounds__(T, (fft_min_blocks<N, T>())) rc_forward_kernel
     if (threadIdx.x == 0) scale[p] = storage_scale(bound);
 }
 
-// N-bin spectrum, M-point transforms (M divides N), G of them per CTA: CTA (p, r0)
-// gives the bins (L N / M) i + r of the phases r = G r0 .. G r0 + G - 1, r < L N / M,
-// each the M-point inverse of the spectrum times its ramp folded modulo M.  The
-// G phases' bins are neighbours in the row, and the last stage's lanes store
-// them together.
-// points between the arrays: in the last stage a half-warp loads 16 / G points of
-// each, from disjoint banks
+// Points between the arrays of a CTA's G phases: in the last stage a half-warp loads
+// 16 / G points of each, from disjoint banks.
 template <int G>
 constexpr int group_pad = G > 1 ? 16 / G : 0;
 // The ramp factors into two levels (per thread, per phase) where every first-stage
@@ -131,6 +126,11 @@ constexpr int kStagedTable = 256 + 16;  // entries at 256 points and 16x
 __device__ __forceinline__ int tslot(int i) { return i + (i >> 3); }
 constexpr int kStagedSlots = kStagedTable + kStagedTable / 8;
 
+// N-bin spectrum, M-point transforms (M divides N), G of them per CTA: CTA (p, r0)
+// gives the bins (L N / M) i + r of the phases r = G r0 .. G r0 + G - 1, r < L N / M,
+// each the M-point inverse of the spectrum times its ramp folded modulo M.  The
+// G phases' bins are neighbours in the row, and the last stage's lanes store
+// them together.
 template <int N, int M, int T, int G, int STORE, bool STAGED>
 __global__ void __launch_bounds__(G *T, (fft_min_blocks<G * M, G * T>()))
     rc_inverse_kernel(int L, int nbins, const float2 *__restrict__ spec, const float2 *__restrict__ etab,
